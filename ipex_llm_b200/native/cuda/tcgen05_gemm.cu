@@ -29,6 +29,7 @@
 #include <stdint.h>
 
 #include "common/utils.cuh"
+#include "lowbit_expand.cuh"
 #include "tcgen05_common.cuh"
 
 namespace {
@@ -78,119 +79,6 @@ struct GemmArgs {
   // M / m_tiles given at launch are the upper bound that sized the grid.
   const int* m_range;
 };
-
-__device__ __forceinline__ int pair_row(int r) { return (r & 7) * 2 + (r >> 3); }
-
-__device__ __forceinline__ float act_apply(float g, int act) {
-  if (act == 1) return g / (1.0f + __expf(-g));
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 0.5f * g * (1.0f + tanhf(k0 * (g + k1 * g * g * g)));
-}
-
-// ------------------------------------------------------------------------------------------------------------------
-// two-lane arithmetic in the activation dtype
-// ------------------------------------------------------------------------------------------------------------------
-template <typename T> struct V2;
-template <> struct V2<__half> {
-  using type = __half2;
-  static __device__ __forceinline__ type bits(uint32_t u) { return *reinterpret_cast<type*>(&u); }
-  static __device__ __forceinline__ uint32_t raw(type v) { return *reinterpret_cast<uint32_t*>(&v); }
-  static __device__ __forceinline__ type splat(float f) { return __float2half2_rn(f); }
-  static constexpr uint32_t kMagic = 0x64006400u;  // 1024 + q
-  static constexpr float kMagicBase = 1024.f;
-};
-template <> struct V2<__nv_bfloat16> {
-  using type = __nv_bfloat162;
-  static __device__ __forceinline__ type bits(uint32_t u) { return *reinterpret_cast<type*>(&u); }
-  static __device__ __forceinline__ uint32_t raw(type v) { return *reinterpret_cast<uint32_t*>(&v); }
-  static __device__ __forceinline__ type splat(float f) { return __float2bfloat162_rn(f); }
-  static constexpr uint32_t kMagic = 0x43004300u;  // 128 + q
-  static constexpr float kMagicBase = 128.f;
-};
-
-// Per-(row, scale group) constants of the dequantizer, already in the two-lane type.
-template <typename T>
-struct Scale {
-  typename V2<T>::type d, m;
-};
-
-// 8 codes of one 32-bit word (4-bit families) -> 8 values in k order, packed as 4 x two-lane.
-// int4 words hold element k in nibble {0,4,1,5,2,6,3,7}[k]: (w >> 4i) & 0x000F000F is the pair (2i, 2i+1).
-template <typename T, int WF>
-__device__ __forceinline__ uint4 expand4(uint32_t w, const Scale<T>& sc, const uint32_t* lut2) {
-  using V = V2<T>;
-  uint32_t r[4];
-  if constexpr (WF == WF_LUT4) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t pair = lut2[(w >> (8 * i)) & 0xFFu];  // (lut[lo nibble], lut[hi nibble]) in T
-      r[i] = V::raw(__hmul2(V::bits(pair), sc.d));
-    }
-  } else {
-    const typename V::type off = V::splat(V::kMagicBase + (WF == WF_SYM_INT4 ? 8.f : 0.f));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t t = ((w >> (4 * i)) & 0x000F000Fu) | V::kMagic;
-      const typename V::type q = __hsub2(V::bits(t), off);  // exact: small integers
-      r[i] = V::raw(WF == WF_SYM_INT4 ? __hmul2(q, sc.d) : __hfma2(q, sc.d, sc.m));
-    }
-  }
-  return make_uint4(r[0], r[1], r[2], r[3]);
-}
-
-// Exponent re-bias for fp8 -> 16-bit float by bit placement: the fp8 byte goes to the top of the 16-bit lane, the
-// 7 magnitude bits are shifted down into the wider exponent field, and the missing 2^delta is folded into the
-// scale.  Works for denormals too (both formats are linear there).
-template <typename T, int WF> struct Fp8Place;
-// `pre` (a power of two, applied to the placed value first) keeps the scale out of fp16's denormal range: e5m2
-// codes reach 57344, so their scales are ~1e-6; codes below 2^-12 of full range may flush, which is far under
-// the format's own resolution.
-template <> struct Fp8Place<__half, WF_FP8_E4M3> {
-  static constexpr int sh = 1; static constexpr float mul = 256.f; static constexpr float pre = 1.f;
-};
-template <> struct Fp8Place<__half, WF_FP8_E5M2> {
-  static constexpr int sh = 0; static constexpr float mul = 4096.f; static constexpr float pre = 1.f / 4096.f;
-};
-template <> struct Fp8Place<__nv_bfloat16, WF_FP8_E4M3> {
-  static constexpr int sh = 4; static constexpr float mul = 1.329227995784916e36f /* 2^120 */;
-  static constexpr float pre = 1.f;
-};
-template <> struct Fp8Place<__nv_bfloat16, WF_FP8_E5M2> {
-  static constexpr int sh = 3; static constexpr float mul = 5.192296858534828e33f /* 2^112 */;
-  static constexpr float pre = 1.f;
-};
-
-// 8 bytes (two words) of an 8-bit family -> 8 values.
-template <typename T, int WF>
-__device__ __forceinline__ uint4 expand8(uint32_t w0, uint32_t w1, const Scale<T>& sc) {
-  using V = V2<T>;
-  uint32_t r[4];
-  const uint32_t ws[2] = {w0, w1};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t w = ws[i >> 1];
-    if constexpr (WF == WF_INT8) {
-      // (1024 + (b ^ 0x80)) - 1152 = signed value, exact in fp16
-      const uint32_t t = __byte_perm(w, 0x64646464u, (i & 1) ? 0x4342 : 0x4140) ^ 0x00800080u;
-      const __half2 q = __hsub2(V2<__half>::bits(t), __float2half2_rn(1152.f));
-      if constexpr (std::is_same<T, __half>::value) {
-        r[i] = V::raw(__hmul2(q, sc.d));
-      } else {
-        const float2 f = __half22float2(q);
-        r[i] = V::raw(__hmul2(__floats2bfloat162_rn(f.x, f.y), sc.d));
-      }
-    } else {
-      using P = Fp8Place<T, WF>;
-      const uint32_t t = __byte_perm(w, 0u, (i & 1) ? 0x3424 : 0x1404);  // bytes to the top of each 16-bit lane
-      uint32_t b = t;
-      if constexpr (P::sh != 0) b = (t & 0x80008000u) | ((t >> P::sh) & (0x7F007F00u >> P::sh));
-      typename V::type val = V::bits(b);
-      if constexpr (P::pre != 1.f) val = __hmul2(val, V::splat(P::pre));
-      r[i] = V::raw(__hmul2(val, sc.d));
-    }
-  }
-  return make_uint4(r[0], r[1], r[2], r[3]);
-}
 
 template <int WF> struct Fam {
   static constexpr bool dense = WF == WF_F16 || WF == WF_BF16;
@@ -708,6 +596,25 @@ int sm_count() {
 // Token tile the kernels use for M tokens.
 IPEX_API int ipex_gemm_tcgen05_token_tile(int M) { return M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256)); }
 
+// gemm_pair_tcgen05.cu: the same products on pairs of SMs.
+IPEX_API int ipex_gemm_pair_tcgen05(const void* x, const void* w, void* out, const void* bias, const void* residual,
+                                    const float* lut, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo,
+                                    int64_t ldr, int wf, int act, int dtype, int bt, int* err, void* stream);
+
+// Token tile of the pair kernel for this product, 0 where the kernel of this file keeps it.  Up to 64 tokens its narrower
+// tiles (32, 64) do less work on padding.  Above, the pair wins at every size measured (int4, K = 4096: 128 x 4096 61.5 ->
+// 37 us, 128 x 12288 62 -> 41, 1024 x 4096 59 -> 31, 1024 x 12288 138 -> 78, 4096 x 22016 788 -> 495; dense fp16 1024 x
+// 12288 96 -> 81).  Between its tiles the count of waves decides: a k block of 128 tokens costs 0.77 of one of 256 with
+// packed weights (the dequantizers' share does not shrink), 0.6 with dense ones.
+static int pair_tile(int M, int N, bool dense, const void* w) {
+  if (M <= 64 || (!dense && (reinterpret_cast<uintptr_t>(w) & 31))) return 0;
+  const int pairs = sm_count() / 2;
+  if (pairs < 1) return 0;
+  const int64_t nt = (N + 255) / 256;
+  const int64_t w256 = ((M + 255) / 256 * nt + pairs - 1) / pairs, w128 = ((M + 127) / 128 * nt + pairs - 1) / pairs;
+  return (dense ? 0.6 : 0.77) * (double)w128 < (double)w256 ? 128 : 256;
+}
+
 // out[M,N] = x[M,K] . w[N,K]^T (+ bias[N]) (+ residual[M,N]).  x, w, out, bias, residual share one 16-bit dtype.
 // Row strides (elements): ldx, ldw multiples of 8 (TMA wants 16-byte strides); x and w 16-byte aligned.
 // Returns a cudaError_t, or -1 when the driver's tensor-map encoder is unavailable / rejects the arguments.
@@ -730,6 +637,9 @@ IPEX_API int ipex_gemm_tcgen05_act(const void* x, const void* w, void* out, cons
   if (act != 0 && (residual != nullptr || (N % 32) != 0)) return (int)cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15)) return (int)cudaErrorInvalidValue;
   if (dtype != DT_F16 && dtype != DT_BF16) return (int)cudaErrorInvalidValue;
+  if (const int pt = pair_tile(M, N, true, w))
+    return ipex_gemm_pair_tcgen05(x, w, out, bias, residual, nullptr, M, N, K, ldx, ldw, ldo, ldr, WF_F16, act, dtype, pt,
+                                  err, stream);
   const int bt = ipex_gemm_tcgen05_token_tile(M);
   const CUtensorMapDataType tdt = dtype == DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUtensorMap tw, tx;
@@ -757,6 +667,9 @@ IPEX_API int ipex_gemm_lowbit_tcgen05(const void* x, const void* w, void* out, c
   if (dtype != DT_F16 && dtype != DT_BF16) return (int)cudaErrorInvalidValue;
   if (act != 0 && (residual != nullptr || (N % 32) != 0)) return (int)cudaErrorInvalidValue;
   if (wf == WF_LUT4 && lut == nullptr) return (int)cudaErrorInvalidValue;
+  if (wf < WF_SYM_INT4 || wf > WF_INT8) return (int)cudaErrorInvalidValue;
+  if (const int pt = pair_tile(M, N, false, w))
+    return ipex_gemm_pair_tcgen05(x, w, out, bias, residual, lut, M, N, K, ldx, 0, ldo, ldr, wf, act, dtype, pt, err, stream);
   const int bt = ipex_gemm_tcgen05_token_tile(M);
   const CUtensorMapDataType tdt = dtype == DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUtensorMap tx;
