@@ -38,9 +38,7 @@ def quantize_to_device_layout(w: torch.Tensor, qtype: int, out: torch.Tensor = N
         raise ValueError(f"in_features {cols} is not a multiple of the {block}-wide block")
     nbytes = device_nbytes(rows, cols, qtype)
     if out is None:
-        out = torch.zeros(nbytes, dtype=torch.uint8, device=w.device)
-    else:
-        out.zero_()
+        out = torch.empty(nbytes, dtype=torch.uint8, device=w.device)       # the kernel writes every byte, padding too
     wf, lut_kind = _GPU_QTYPES[qtype]
     rc = lib.ipex_quantize_to_tiles(ptr(w2), ptr(out), rows, cols, w2.stride(0), wf, lut_kind,
                                     api.dtype_code(w2.dtype), current_stream())

@@ -245,8 +245,16 @@ class FP4Params(torch.nn.Parameter):
         """Pack ``data`` (a float weight) into canonical blocks on the CPU (or shapes only on meta)."""
         if self.quantized:
             return self
-        w = self.data.contiguous().float()
+        w = self.data.contiguous()
         qtype = self.qtype
+        meta = device is not None and str(device) == "meta"
+        # the GPU quantizer reads 16-bit weights itself; everything else works on fp32
+        direct = False
+        if w.is_cuda and not meta and self.imatrix is None and w.dtype in (torch.float16, torch.bfloat16):
+            from ..ops import cuda_quant
+            direct = cuda_quant.can_quantize_on_gpu(qtype)
+        if not direct:
+            w = w.float()
         if qtype == qt.MOFQ4:
             qtype = qt.SYM_INT4 if self.ggml_mse(w, qt.SYM_INT4, device) <= self.ggml_mse(w, qt.FP4, device) \
                 else qt.FP4
@@ -255,7 +263,6 @@ class FP4Params(torch.nn.Parameter):
                 else qt.FP8E4
         self.qtype = qtype
         self._shape = w.shape
-        meta = device is not None and str(device) == "meta"
         if not meta and w.is_cuda and iq.is_iq(qtype):
             # the code-book search is tensor code: it runs where the weight is, and block order is also what the
             # device keeps for these formats

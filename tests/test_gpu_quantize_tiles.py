@@ -1,0 +1,43 @@
+"""The GPU quantizer and its inverse at the edges of their tiles (16 rows x 128 k), against the host library."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+NAMES = ["sym_int4", "asym_int4", "nf4", "fp4", "fp8_e4m3", "fp8_e5m2", "sym_int8"]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 64), (16, 128), (17, 192), (31, 320), (80, 1088), (2500, 128)])
+@pytest.mark.parametrize("name", NAMES)
+def test_pack_and_expand(name, shape, dtype):
+    from ipex_llm_b200.ops.cuda_ops import dequantize_device
+    from ipex_llm_b200.ops.cuda_quant import quantize_to_device_layout
+    from ipex_llm_b200.quant import qtypes as qt
+    from ipex_llm_b200.quant.params import FP4Params, ggml_convert_fp32, ggml_convert_qtype
+    N, K = shape
+    if name.startswith("fp8"):
+        K = (K + 127) // 128 * 128
+    q = qt.qtype_from_name(name)
+    g = torch.Generator().manual_seed(N * 7 + K)
+    w = (torch.randn(N, K, generator=g) * 0.02).to(dtype)
+    w[0, :64] = 0.0                                             # a block without a scale
+    dev = w.cuda()
+    packed = quantize_to_device_layout(dev, q)
+    # rows that are neither aligned to 16 bytes nor packed one after another take the element-wise loads: same bytes
+    wide = torch.zeros(N, K + 3, dtype=dtype, device="cuda")
+    wide[:, 1:K + 1] = dev
+    assert torch.equal(packed, quantize_to_device_layout(wide[:, 1:K + 1], q))
+    # a used buffer is overwritten whole, padding included
+    assert torch.equal(packed, quantize_to_device_layout(dev, q, out=torch.full_like(packed, 0xA5)))
+    assert torch.equal(packed, FP4Params(dev, requires_grad=False, quantized=False, qtype=q).to("cuda").data)
+    back = dequantize_device(packed, (N, K), q, torch.float32).cpu()
+    host = ggml_convert_fp32(ggml_convert_qtype(w.float().contiguous(), q).view(torch.uint8), w.shape, w.numel(), q)
+    if name.startswith("fp8"):
+        # ties of the two roundings to fp8 may fall to either neighbour: half a unit of three (two) mantissa bits each
+        step = w.float().abs() * (2.0 ** -3 if name == "fp8_e4m3" else 2.0 ** -2) + w.float().abs().amax() * 2.0 ** -14
+        assert bool(((back - host).abs() <= step).all())
+    else:
+        assert torch.equal(back, host)
+    for half in (torch.float16, torch.bfloat16):
+        assert torch.equal(dequantize_device(packed, (N, K), q, half).cpu(), back.to(half))
