@@ -56,6 +56,60 @@ __global__ void norm_kernel(const T* __restrict__ x, const T* __restrict__ w, co
   }
 }
 
+// RMSNorm of rows whose length is a multiple of 8 and at most 16384: the row stays in registers, 16 bytes an access.  Bounded
+// by memory (one read, one write).  PAIRS: the 32-bit result as two 16-bit rows, the rounded value (row 2r) and what that left
+// over (row 2r + 1), for products that take both.
+template <typename T, bool PAIRS>
+__global__ void __launch_bounds__(512) rms_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
+                                                       int H, float eps, float w_offset) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float red[16];
+  const int tid = threadIdx.x, nt = blockDim.x, nvec = H / 8;
+  const uint4* row = reinterpret_cast<const uint4*>(x + (size_t)blockIdx.x * H);
+  uint4 v[4];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (tid + i * nt >= nvec) break;
+    v[i] = row[tid + i * nt];
+    const T* e = reinterpret_cast<const T*>(&v[i]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float f = DT<T>::to_f(e[j]);
+      ss += f * f;
+    }
+  }
+  ss = warp_sum(ss);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+  for (int i = 0; i < nt / 32; ++i) tot += red[i];
+  const float rstd = rsqrtf(tot / H + eps);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = tid + i * nt;
+    if (c >= nvec) break;
+    uint4 wv = make_uint4(0, 0, 0, 0);
+    if (w != nullptr) wv = reinterpret_cast<const uint4*>(w)[c];
+    const T* e = reinterpret_cast<const T*>(&v[i]);
+    const T* we = reinterpret_cast<const T*>(&wv);
+    __align__(16) T hi[8], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float g = (w != nullptr ? DT<T>::to_f(we[j]) : 1.f) + w_offset;
+      float f = DT<T>::to_f(e[j]) * rstd;
+      if (!PAIRS) f = DT<T>::to_f(DT<T>::from_f(f));   // HF casts the normalised value before the weight multiply
+      f *= g;
+      hi[j] = DT<T>::from_f(f);
+      if (PAIRS) lo[j] = DT<T>::from_f(f - DT<T>::to_f(hi[j]));
+    }
+    uint4* to = reinterpret_cast<uint4*>(y + (size_t)blockIdx.x * (PAIRS ? 2 : 1) * H);
+    to[c] = *reinterpret_cast<const uint4*>(hi);
+    if (PAIRS) to[nvec + c] = *reinterpret_cast<const uint4*>(lo);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------
 // act(gate) * up
 // ------------------------------------------------------------------------------------------------
@@ -277,6 +331,13 @@ IPEX_API int ipex_rms_norm(const void* x, const void* w, const void* residual, v
                            int H, float eps, float w_offset, int dtype, int pdl, void* stream) {
   return by_dtype(dtype, [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
+    if constexpr (sizeof(T) == 2) {
+      // whole 16-byte accesses on every row: 1024 x 4096 fp16 9.6 -> 4.2 us
+      const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y);
+      if (residual == nullptr && H % 8 == 0 && H <= 16384 && (all & 15) == 0)
+        return launch_kernel(rms_rows_kernel<T, false>, dim3((unsigned)rows), dim3(H > 4096 ? 512 : H > 2048 ? 256 : 128), 0,
+                             (cudaStream_t)stream, pdl != 0, (const T*)x, (const T*)w, (T*)y, H, eps, w_offset);
+    }
     int threads = H >= 2048 ? 512 : 256;
     size_t smem = (size_t)(H + 64) * sizeof(float);
     auto kern = norm_kernel<T, false>;
@@ -285,6 +346,23 @@ IPEX_API int ipex_rms_norm(const void* x, const void* w, const void* residual, v
                          (const T*)x, (const T*)w, (const T*)nullptr, (const T*)residual, (T*)y, (T*)res_out, H, eps,
                          w_offset);
   });
+}
+
+// y [2 rows, H]: value and remainder of every normalised row (rms_rows_kernel).  H a multiple of 8 up to 16384, pointers
+// 16-byte aligned.
+IPEX_API int ipex_rms_norm_pairs(const void* x, const void* w, void* y, int64_t rows, int H, float eps, float w_offset,
+                                 int dtype, int pdl, void* stream) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y);
+  if (rows < 1 || H < 8 || H % 8 != 0 || H > 16384 || (all & 15) != 0) return (int)cudaErrorInvalidValue;
+  const dim3 grid((unsigned)rows), block(H > 4096 ? 512 : H > 2048 ? 256 : 128);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (dtype == DT_F16)
+    return (int)launch_kernel(rms_rows_kernel<__half, true>, grid, block, 0, st, pdl != 0, (const __half*)x, (const __half*)w,
+                              (__half*)y, H, eps, w_offset);
+  if (dtype == DT_BF16)
+    return (int)launch_kernel(rms_rows_kernel<__nv_bfloat16, true>, grid, block, 0, st, pdl != 0, (const __nv_bfloat16*)x,
+                              (const __nv_bfloat16*)w, (__nv_bfloat16*)y, H, eps, w_offset);
+  return (int)cudaErrorInvalidValue;
 }
 
 IPEX_API int ipex_layer_norm(const void* x, const void* w, const void* b, void* y, int64_t rows, int H, float eps,

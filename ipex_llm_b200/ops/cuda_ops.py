@@ -99,6 +99,15 @@ def gemv_lowbit(x: torch.Tensor, w_data: torch.Tensor, qtype: int, N: int, K: in
     if out is None:
         out = torch.empty((M, n_out), dtype=x.dtype, device=x.device)
     lut = lut_for(qtype, x.device) if wf == api.WF_LUT4 else None
+    if M > 4 and K > 8192 and K % 128 == 0 and N % 16 == 0 and norm_weight is None and act == 0 and \
+            wf not in (api.WF_F16, api.WF_BF16) and x.dtype in (torch.float16, torch.bfloat16) and \
+            out.dtype == x.dtype and out.stride(1) == 1 and _GEMV_IMPL == "stream":
+        # five to eight long rows do not fit beside the rings of the kernels below, which then stream the weights twice or
+        # leave the rings: 4096 x 11008 at 8 rows, int4 33.8 -> 18.8 us, fp8 36.6 -> 25.1, nf4 143 -> 27.6
+        from . import tcgen05_gemm
+        if tcgen05_gemm.few_exact(wf, x.dtype, M) and \
+                tcgen05_gemm.gemm_few(x, w_data, N, K, out, wf, lut=lut, bias=bias, residual=residual, pdl=pdl and _USE_PDL):
+            return out
     if _GEMV_IMPL == "stream" and wf in (api.WF_SYM_INT4, api.WF_FP8_E4M3) and x.stride(0) % 8 == 0 and \
             getattr(lib, "ipex_gemv_lowbit_stream", None) is not None:
         # warp-private rings, one tensor-core instruction per 512 weights for up to four tokens
@@ -298,6 +307,17 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, offset: float = 
     rc = lib.ipex_rms_norm(ptr(xc), ptr(w), ptr(residual), ptr(out), ptr(residual_out), rows, H, eps, offset, _dt(xc),
                            int(pdl and _USE_PDL), current_stream())
     api.check(rc, "rms_norm")
+    return out
+
+
+def rms_norm_pairs(x: torch.Tensor, weight: torch.Tensor, eps: float, offset: float = 0.0, pdl: bool = False) -> torch.Tensor:
+    """RMSNorm of ``x [rows, H]`` in 32 bits, as ``[2 * rows, H]`` of x's type: every row's rounded values, then what the
+    rounding left over (together twice the type's precision)."""
+    rows, H = x.shape
+    out = torch.empty((2 * rows, H), dtype=x.dtype, device=x.device)
+    rc = cuda_lib().ipex_rms_norm_pairs(ptr(x), ptr(weight), ptr(out), rows, H, eps, offset, _dt(x), int(pdl and _USE_PDL),
+                                        current_stream())
+    api.check(rc, "rms_norm_pairs")
     return out
 
 

@@ -98,6 +98,37 @@ def gemm_lowbit(x: torch.Tensor, w_data: torch.Tensor, qtype: int, N: int, K: in
 
 
 
+FEW_MAX_ROWS = 64      # rows of x (two per token when it comes in pairs) that gemm_few takes
+
+
+def few_exact(wf: int, dtype, rows: int) -> bool:
+    """Whether ``gemm_few`` multiplies by the codes of this format without rounding them (``rows`` of x up to 32, or pairs):
+    then it is at least as precise as the kernels for one to eight rows.  A code book's values round to bf16, a format with
+    minima is expanded to 16 bits."""
+    if wf == api.WF_ASYM_INT4 or (wf == api.WF_LUT4 and dtype != torch.float16):
+        return False
+    return rows <= 32
+
+
+def gemm_few(x: torch.Tensor, w_data: torch.Tensor, N: int, K: int, out: torch.Tensor, wf: int, lut: torch.Tensor = None,
+             bias: torch.Tensor = None, residual: torch.Tensor = None, act: int = 0, pairs: bool = False,
+             pdl: bool = False) -> bool:
+    """``x @ dequant(w).T`` for few rows into ``out`` (see native/cuda/gemm_few_tcgen05.cu); ``pairs``: ``x`` holds value and
+    remainder of every token in turn (``cuda_ops.rms_norm_pairs``).  False when the operands do not suit the kernel."""
+    lib = cuda_lib()
+    M = out.shape[0]
+    if x.shape[0] > FEW_MAX_ROWS or x.stride(1) != 1 or x.stride(0) % 8 != 0 or x.data_ptr() % 16 != 0 or \
+            w_data.data_ptr() % 32 != 0 or (residual is not None and residual.stride(1) != 1):
+        return False
+    rc = lib.ipex_gemm_few_tcgen05(ptr(x), ptr(w_data), ptr(out), ptr(bias), ptr(residual), ptr(lut), M, N, K, x.stride(0),
+                                   out.stride(0), residual.stride(0) if residual is not None else 0, wf, int(act), int(pairs),
+                                   api.dtype_code(x.dtype), int(pdl), ptr(_err(x.device)), current_stream())
+    if rc == -1:
+        raise RuntimeError("ipex_llm_b200: the driver's tensor-map encoder rejected the GEMM operands")
+    api.check(rc, "gemm_few_tcgen05")
+    return True
+
+
 def gemm_lowbit_ar(x: torch.Tensor, w_data: torch.Tensor, qtype: int, N: int, K: int, comm, out: torch.Tensor = None,
                    bias: torch.Tensor = None, residual: torch.Tensor = None, wf: int = None) -> torch.Tensor:
     """Row-parallel projection of a tensor-parallel model: ``sum_over_ranks(x_r @ dequant(W_r).T) (+ bias)

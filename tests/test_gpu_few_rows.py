@@ -1,0 +1,119 @@
+"""The product for few rows (a tile's k shared by a cluster) at the edges of its tiles, and the norm in front of it, against
+float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+U = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+# (M, N, K): one to 64 rows on both sides of every column count; fewer k tiles than CTAs in a cluster, a share that is not the
+# same for all of them; fewer weight rows than a tile, tiles in a second round with a ragged last one
+SHAPES = [(1, 16, 128), (5, 144, 384), (16, 272, 640), (17, 400, 1152), (32, 128, 512), (33, 5008, 256), (64, 1040, 896)]
+
+
+def _weights(name, N, K, dtype, g):
+    from ipex_llm_b200.ops import cuda_ops, cuda_quant
+    from ipex_llm_b200.quant import qtypes as qt
+    q = qt.qtype_from_name(name)
+    packed = cuda_quant.quantize_to_device_layout((torch.randn(N, K, device="cuda", generator=g) * 0.05).to(dtype), q)
+    return q, packed, cuda_ops.dequantize_device(packed, (N, K), q, torch.float32).double()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("name", ["sym_int4", "asym_int4", "nf4", "fp8_e4m3", "fp8_e5m2", "sym_int8"])
+def test_few_rows(name, shape, dtype):
+    from ipex_llm_b200.ops import cuda_ops, tcgen05_gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    q, packed, w = _weights(name, N, K, dtype, g)
+    wf = cuda_ops.QTYPE_TO_WF[q]
+    xf = torch.randn(M, K, device="cuda", generator=g)
+    bias = torch.randn(N, device="cuda", generator=g).to(dtype)
+    res = torch.randn(M, N, device="cuda", generator=g).to(dtype)
+    for pairs in (False, True):
+        if pairs and 2 * M > tcgen05_gemm.FEW_MAX_ROWS:
+            continue
+        hi = xf.to(dtype)
+        lo = (xf - hi.float()).to(dtype)
+        x = torch.stack([hi, lo], 1).reshape(2 * M, K) if pairs else hi
+        xd = hi.double() + lo.double() if pairs else hi.double()
+        run = lambda **kw: tcgen05_gemm.gemm_few(x, packed, N, K, kw.pop("out"), wf, lut=cuda_ops.lut_for(q, x.device),  # noqa: E731
+                                                 pairs=pairs, **kw)
+        out, full = (torch.full((M, N), float("nan"), dtype=dtype, device="cuda") for _ in range(2))
+        assert run(out=out) and run(out=full, bias=bias, residual=res)
+        torch.cuda.synchronize()
+        cuda_ops.check_error_flag(x.device)
+        mag, ref = xd.abs() @ w.abs().t(), xd @ w.t()
+        # roundings of a weight on its way (half a unit each): none where the codes are multiplied, the value of a code book,
+        # and value, scale and product (a minimum beside them: bounded by its block's largest weight) where weights are expanded
+        codes = pairs or M <= 32 or name.startswith("fp8")
+        roundings = 8 if name == "asym_int4" else (1 if name == "nf4" else 0) if codes else 3
+        bound = mag * (roundings * U[dtype] + K * 2.0 ** -23) + ref.abs() * U[dtype] + 1e-6
+        assert bool(((out.double() - ref).abs() <= bound).all())
+        ref2 = ref + bias.double() + res.double()
+        assert bool(((full.double() - ref2).abs() <= bound + (ref2.abs() + 4.0) * U[dtype]).all())
+        again = torch.empty_like(out)
+        run(out=again)
+        assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("pairs", [False, True])
+@pytest.mark.parametrize("shape", [(9, 288, 256), (24, 4128, 512)])
+def test_few_rows_gated(shape, pairs):
+    from ipex_llm_b200.ops import cuda_ops, tcgen05_gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q, packed, w = _weights("sym_int4", N, K, torch.float16, g)
+    x = torch.randn(2 * M if pairs else M, K, device="cuda", generator=g).half()
+    xd = x.double().view(M, 2, K).sum(1) if pairs else x.double()
+    out = torch.empty(M, N // 2, dtype=torch.float16, device="cuda")
+    assert tcgen05_gemm.gemm_few(x, packed, N, K, out, cuda_ops.QTYPE_TO_WF[q], act=1, pairs=pairs)
+    torch.cuda.synchronize()
+    cuda_ops.check_error_flag(x.device)
+    t = (xd @ w.t()).view(M, N // 32, 2, 16)
+    ref = (torch.nn.functional.silu(t[:, :, 0]) * t[:, :, 1]).reshape(M, N // 2)
+    # an approximate exponential (2^-10 of the gate) and the rounding of the result
+    assert bool(((out.double() - ref).abs() <= ref.abs() * U[torch.float16] + 2.0 ** -10 * t.abs().amax() ** 2 / 8).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("H", [8, 264, 2048, 4096, 13824, 16384])
+def test_rms_norm_rows(H, dtype):
+    from ipex_llm_b200.ops import cuda_ops
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x = torch.randn(5, H, device="cuda", generator=g).to(dtype)
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).to(dtype)
+    ref = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    pair = cuda_ops.rms_norm_pairs(x, w, 1e-5).view(5, 2, H).double()
+    # the remainder has the type's relative precision, down to its smallest step
+    assert bool(((pair.sum(1) - ref).abs() <= ref.abs() * (U[dtype] ** 2 * 2 + 2.0 ** -20) + 2.0 ** -24).all())
+    one = cuda_ops.rms_norm(x, w, 1e-5).double()
+    assert bool(((one - ref).abs() <= ref.abs() * (2.5 * U[dtype]) + 1e-7).all())    # value and product are rounded
+
+
+@pytest.mark.parametrize("batch", [9, 20, 32])
+def test_decode_steps_of_a_batch(batch):
+    """Steps of a batch against the same sequences decoded eight at a time."""
+    from transformers import LlamaConfig
+    from ipex_llm_b200.engine.decoder_engine import DecoderEngine
+    from ipex_llm_b200.transformers import AutoModelForCausalLM
+    cfg = LlamaConfig(hidden_size=512, intermediate_size=1408, num_hidden_layers=2, num_attention_heads=4,
+                      num_key_value_heads=4, vocab_size=1024, max_position_embeddings=512, tie_word_embeddings=False)
+    model = AutoModelForCausalLM.from_config(cfg, load_in_low_bit="sym_int4", device="cuda:0", torch_dtype=torch.float16)
+    ids = torch.randint(0, 1024, (batch, 24), device="cuda", generator=torch.Generator(device="cuda").manual_seed(batch))
+
+    def steps(rows):
+        eng = DecoderEngine(model, max_batch=rows.shape[0], max_len=256, kv_fp8=False)
+        eng.prefill(rows)
+        out = []
+        for i in range(3):
+            eng.tokens[:rows.shape[0]] = rows[:, i]
+            eng.decode_step(rows.shape[0])
+            out.append(eng.logits[:rows.shape[0]].double().clone())
+        return torch.stack(out)
+
+    whole = steps(ids)
+    parts = torch.cat([steps(ids[s:s + 8]) for s in range(0, batch, 8)], dim=1)
+    # both round every activation to fp16 about thirty times on the way: 2^-11 each, and no more than a few of them add up
+    assert float((whole - parts).norm() / parts.norm()) < 8 * 2.0 ** -11
