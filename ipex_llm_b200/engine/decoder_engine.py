@@ -323,17 +323,12 @@ class DecoderEngine:
         return out
 
     def _pick_splits(self, B: int) -> int:
-        """KV splits of the decode attention, sized for the context this generation will actually reach (the next
-        power of two above prompt + 256 tokens) rather than for the cache capacity: the kernel divides whatever
-        length it finds by this count, and 2816 tokens of capacity gave a 1024-token prompt 22 splits of 48 tokens
-        where 11 splits are best (Llama-2-7B: 2.00 ms per token against 1.86 ms).  The count is part of the
-        captured graph, so graphs are kept per (batch, splits)."""
+        """KV splits of the decode attention, sized for the context this generation starts from (with 256 tokens to come)
+        rather than for the cache capacity: the kernel divides whatever length it finds by this count.  The count is part
+        of the captured graph, so graphs are kept per (batch, splits)."""
         hint = self._kv_hint if self._kv_hint else self.max_len
-        target = 512
-        while target < hint + 256:
-            target *= 2
-        target = min(target, self.max_len)
-        return cuda_ops.pick_nsplit(B, self.n_kv, target, rows=self.n_heads // self.n_kv)
+        return cuda_ops.attn_splits(B, self.n_kv, min(hint + 256, self.max_len), self.n_heads // self.n_kv, self.hd,
+                                    self.kv_fp8, self.dtype)
 
     def _attention(self, L: _Layer, B: int, Sq: int = 1):
         """Rope + cache append + attention for ``B`` sequences of ``Sq`` new tokens each; rows of the activation

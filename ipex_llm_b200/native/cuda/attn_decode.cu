@@ -16,6 +16,7 @@
 //                  of the last split, and attended to from shared memory (causal among themselves).
 // mode B (module path): the cache already holds every token; q is already rotated.
 #include <cstdlib>
+#include <type_traits>
 
 #include "common/utils.cuh"
 
@@ -83,6 +84,11 @@ struct RawKV {
     }
   }
 
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < kWords; i++) w[i] = 0;
+  }
+
   __device__ __forceinline__ void decode(float (&out)[DPL]) const {
     if constexpr (FP8) {
 #pragma unroll
@@ -138,6 +144,38 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
   const int rg_p2 = row_groups <= 1 ? 1 : (row_groups <= 2 ? 2 : 4);
   const int TS = kAttnWarps / rg_p2;
   const int rg = warp % rg_p2, tsub = warp / rg_p2;
+
+  // ---- cached tokens of this split: the first steps' words are requested before the queries are prepared ----
+  // Software pipeline on the raw cache words, kPF steps deep.  A step is four tokens a warp; kPF steps are one batch whose
+  // scores, maximum and exponentials are worked out together: the online soft-max is a chain of some 600 clocks, which
+  // bounded the walk when every step went through it (64 steps of one head: 27 us, 32-step walks of a kv head with 8 query
+  // heads: 44 us), and is now paid once a batch.  Keys of the next batch are requested as soon as a batch's scores are
+  // known, values when its sums are.
+  using Raw = RawKV<T, FP8, DPL>;
+  constexpr int kStepWords = 2 * Raw::kWords;            // registers one step in flight holds
+  constexpr int kState = 2 * RW * DPL;                   // registers of the q rows and their accumulators
+  constexpr int kBudget = kState <= 64 ? 64 : (kState <= 128 ? 32 : 16);
+  constexpr int kWant = kBudget / kStepWords;
+  constexpr int kPF = kWant >= 4 ? 4 : 2;
+  int chunk = (past + a.nsplit - 1) / a.nsplit;
+  chunk = (chunk + 15) & ~15;
+  const int t0 = split * chunk;
+  const int t1 = min(past, t0 + chunk);
+  const int stride = 4 * TS;
+  const uint8_t* kc = reinterpret_cast<const uint8_t*>(a.kcache);
+  const uint8_t* vc = reinterpret_cast<const uint8_t*>(a.vcache);
+  const int64_t head_off = b * a.c_b + (int64_t)kvh * a.c_h + ds * DPL;
+  Raw kq[kPF], vq[kPF];
+#pragma unroll
+  for (int i = 0; i < kPF; i++) {
+    const int p = t0 + tsub * 4 + i * stride + tg;
+    kq[i].clear();
+    vq[i].clear();
+    if (p < t1) {
+      kq[i].load(kc, head_off + (int64_t)p * a.c_s);
+      vq[i].load(vc, head_off + (int64_t)p * a.c_s);
+    }
+  }
 
   // ---- q rows of this warp, rotated, pre-scaled, in registers ----
   float qr[RW][DPL];
@@ -264,60 +302,74 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
     }
   };
 
-  // ---- cached tokens of this split ----
-  {
-    int chunk = (past + a.nsplit - 1) / a.nsplit;
-    chunk = (chunk + 15) & ~15;
-    const int t0 = split * chunk;
-    const int t1 = min(past, t0 + chunk);
-    const uint8_t* kc = reinterpret_cast<const uint8_t*>(a.kcache);
-    const uint8_t* vc = reinterpret_cast<const uint8_t*>(a.vcache);
-    const int64_t head_off = b * a.c_b + (int64_t)kvh * a.c_h + ds * DPL;
-    // software pipeline on the raw cache words, kPF steps deep: a step's loads are issued kPF steps before the
-    // (serial) online-softmax update consumes them.  One step ahead left every step waiting for most of an L2
-    // round trip (about 1 us per step measured: 59 us for the 32-step walks of one kv head with 8 query heads).
-    using Raw = RawKV<T, FP8, DPL>;
-    constexpr int kStepWords = 2 * Raw::kWords;            // registers one step in flight holds
-    constexpr int kState = 2 * RW * DPL;                   // registers of the q rows and their accumulators
-    constexpr int kBudget = kState <= 64 ? 48 : (kState <= 128 ? 32 : 16);
-    constexpr int kWant = kBudget / kStepWords;
-    constexpr int kPF = kWant >= 4 ? 4 : (kWant >= 2 ? kWant : 2);
-    Raw kq[kPF], vq[kPF];
-    const int stride = 4 * TS;
-    int base = t0 + tsub * 4;
+  for (int base = t0 + tsub * 4; base < t1; base += kPF * stride) {
+    float sc[kPF][RW];
 #pragma unroll
     for (int i = 0; i < kPF; i++) {
-      const int p = base + i * stride + tg;
-      if (p < t1) {
-        kq[i].load(kc, head_off + (int64_t)p * a.c_s);
-        vq[i].load(vc, head_off + (int64_t)p * a.c_s);
+      float kf[DPL];
+      kq[i].decode(kf);
+#pragma unroll
+      for (int r = 0; r < RW; r++) {
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int d = 0; d < DPL; d += 2) {
+          s0 += qr[r][d] * kf[d];
+          s1 += qr[r][d + 1] * kf[d + 1];
+        }
+        sc[i][r] = s0 + s1;
       }
     }
-    while (base < t1) {
+#pragma unroll
+    for (int i = 0; i < kPF; i++) {
+      const int np = base + (kPF + i) * stride + tg;
+      if (np < t1) kq[i].load(kc, head_off + (int64_t)np * a.c_s);
+    }
+#pragma unroll
+    for (int o = 1; o <= 4; o <<= 1)
+#pragma unroll
+      for (int i = 0; i < kPF; i++)
+#pragma unroll
+        for (int r = 0; r < RW; r++) sc[i][r] += __shfl_xor_sync(0xffffffffu, sc[i][r], o);
+    float corr[RW];
+#pragma unroll
+    for (int r = 0; r < RW; r++) {
+      float mn = m[r];
 #pragma unroll
       for (int i = 0; i < kPF; i++) {
-        const int cur = base + i * stride;                 // warp-uniform
-        if (cur < t1) {
-          const int pos = cur + tg;
-          const bool valid = pos < t1;
-          float kf[DPL], vf[DPL];
-          if (valid) {
-            kq[i].decode(kf);
-            vq[i].decode(vf);
-          } else {
-#pragma unroll
-            for (int d = 0; d < DPL; d++) { kf[d] = 0.f; vf[d] = 0.f; }
-          }
-          // the slot is free again: refill it with the step kPF ahead before the softmax update
-          const int np = cur + kPF * stride + tg;
-          if (np < t1) {
-            kq[i].load(kc, head_off + (int64_t)np * a.c_s);
-            vq[i].load(vc, head_off + (int64_t)np * a.c_s);
-          }
-          consume(kf, vf, pos, valid);
+        const int pos = base + i * stride + tg;
+        float s = sc[i][r];
+        if (cap > 0.f) s = cap * tanhf(s * inv_cap_scaled);
+        bool ok = pos < t1 && qpos[r] >= 0;
+        if (ok && causal) {
+          const int limit = causal_base + qpos[r] + 1;
+          ok = pos < limit && (a.window <= 0 || pos >= limit - a.window);
         }
+        sc[i][r] = ok ? s : -INFINITY;
+        mn = fmaxf(mn, sc[i][r]);
       }
-      base += kPF * stride;
+      const float ref = mn == -INFINITY ? 0.f : mn;      // nothing visible yet: every weight is zero
+      corr[r] = __expf(m[r] - ref);
+      l[r] *= corr[r];
+#pragma unroll
+      for (int i = 0; i < kPF; i++) {
+        sc[i][r] = __expf(sc[i][r] - ref);
+        l[r] += sc[i][r];
+      }
+      m[r] = mn;
+#pragma unroll
+      for (int d = 0; d < DPL; d++) acc[r][d] *= corr[r];
+    }
+#pragma unroll
+    for (int i = 0; i < kPF; i++) {
+      float vf[DPL];
+      vq[i].decode(vf);
+      const int np = base + (kPF + i) * stride + tg;
+      if (np < t1) vq[i].load(vc, head_off + (int64_t)np * a.c_s);
+      else vq[i].clear();
+#pragma unroll
+      for (int r = 0; r < RW; r++)
+#pragma unroll
+        for (int d = 0; d < DPL; d++) acc[r][d] += sc[i][r] * vf[d];
     }
   }
   // ---- new tokens (mode A, last split) from shared memory ----
@@ -511,6 +563,34 @@ IPEX_API int64_t ipex_attn_decode_counter_ints(int B, int Hkv, int G, int Sq) {
   const int rows_total = G * Sq;
   const int nrb = (rows_total + kMaxRows - 1) / kMaxRows;
   return (int64_t)B * Hkv * nrb;
+}
+
+// CTAs of a launch with `rows` query rows per kv head (group x positions) that one SM holds at a time; 0 where the head size
+// or type is not taken.
+IPEX_API int ipex_attn_decode_ctas_per_sm(int D, int rows, int fp8_kv, int dtype) {
+  auto ask = [&](auto* tag, auto fp8, auto d) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    constexpr bool kF = decltype(fp8)::value;
+    constexpr int kD = decltype(d)::value;
+    const int r = min(kMaxRows, rows);
+    const int rw = r <= 1 ? 1 : (r <= 8 && !(r > 4 && wide_rows())) ? 2 : 4;
+    const void* k = rw == 1   ? (const void*)attn_decode_kernel<T, kF, kD, 1>
+                    : rw == 2 ? (const void*)attn_decode_kernel<T, kF, kD, 2>
+                              : (const void*)attn_decode_kernel<T, kF, kD, 4>;
+    int n = 0;
+    const size_t sm = (size_t)(2 * kD + kAttnWarps * rw * (kD + 2) + 33 * kMaxRows) * sizeof(float);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kAttnThreads, sm) == cudaSuccess ? n : 0;
+  };
+  auto by_d = [&](auto* tag, auto fp8) {
+    switch (D) {
+      case 64: return ask(tag, fp8, std::integral_constant<int, 64>());
+      case 128: return ask(tag, fp8, std::integral_constant<int, 128>());
+      case 256: return ask(tag, fp8, std::integral_constant<int, 256>());
+      default: return 0;
+    }
+  };
+  auto by_kv = [&](auto* tag) { return fp8_kv ? by_d(tag, std::true_type()) : by_d(tag, std::false_type()); };
+  return dtype == DT_F16 ? by_kv((__half*)nullptr) : dtype == DT_BF16 ? by_kv((__nv_bfloat16*)nullptr) : 0;
 }
 
 // See AttnArgs for the meaning of the arguments.  `counters` must be zero before the first call; the kernel

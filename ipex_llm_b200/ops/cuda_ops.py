@@ -8,6 +8,7 @@ fallback on a GPU.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 
@@ -455,6 +456,27 @@ def pick_nsplit(B: int, Hkv: int, kv_len: int, n_sm: int = 148, rows: int = 1) -
     return int(max(1, min(by_len, 128)))
 
 
+@functools.lru_cache(maxsize=None)
+def _attn_ctas_per_sm(head_dim: int, rows: int, fp8: bool, dtype_code: int) -> int:
+    return max(1, int(cuda_lib().ipex_attn_decode_ctas_per_sm(head_dim, min(rows, 16), int(fp8), dtype_code)))
+
+
+def attn_splits(B: int, Hkv: int, kv_len: int, rows: int, head_dim: int, fp8: bool, dtype: torch.dtype) -> int:
+    """KV splits of a decode attention over ``B`` sequences of ``Hkv`` kv heads with ``rows`` q rows each (GQA group x query
+    length).  As many as the GPU holds CTAs of at once (a second wave doubles the launch: 8 sequences x 32 heads of 517
+    tokens 17 us at 2 splits, 24 at 4), and no walk shorter than it takes to pay for handing its sums over: 160 tokens, or
+    512 where the heads alone fill the GPU (8 x 517 tokens 15.9 us whole, 17.3 in two; 8 x 2048 49 and 39; one sequence of
+    1024 11.3 us at 8 splits, 12.3 at 11, 13.1 at 3).  ``pick_nsplit``'s rule, which knows the walk's length only, where its
+    switches ask for it."""
+    if "IPEX_LLM_ATTN_STEPS" in os.environ or "IPEX_LLM_ATTN_MIN_CTAS" in os.environ:
+        return pick_nsplit(B, Hkv, kv_len, rows=rows)
+    heads = B * Hkv * -(-max(1, rows) // 16)
+    wave = 148 * _attn_ctas_per_sm(head_dim, max(1, rows), bool(fp8), api.dtype_code(dtype)) // heads
+    n = min(wave, kv_len // (512 if heads >= 148 else 160))
+    # a captured step keeps its count: few different ones, so that prompts of similar length share a graph
+    return max(c for c in (1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128) if c <= max(1, n))
+
+
 _attn_ws_retired = []
 
 
@@ -508,7 +530,7 @@ def sdpa_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask, scale: 
         q = q.contiguous()
     out = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device)
     G = Hq // Hkv
-    nsplit = pick_nsplit(B, Hkv, Skv, rows=G * Sq)
+    nsplit = attn_splits(B, Hkv, Skv, G * Sq, D, fp8, q.dtype)
     floats = lib.ipex_attn_decode_scratch_floats(B, Hkv, G, Sq, D, nsplit)
     ints = lib.ipex_attn_decode_counter_ints(B, Hkv, G, Sq)
     scratch, counters = attn_workspace(q.device, floats, ints)

@@ -1,0 +1,49 @@
+"""The decode attention's walk over cached tokens at the edges of its batches and splits, against float64."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads", [(4, 4, 1), (8, 2, 1), (8, 2, 3), (16, 1, 1)])     # one, four, twelve and sixteen rows a head
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("kind", ["half", "bf16", "e5m2"])
+def test_walk(kind, D, heads, monkeypatch):
+    from ipex_llm_b200.ops import cuda_ops
+    Hq, Hkv, Sq = heads
+    dtype = torch.bfloat16 if kind == "bf16" else torch.float16
+    u = 2.0 ** -8 if kind == "bf16" else 2.0 ** -11
+    g = torch.Generator(device="cuda").manual_seed(D + Hq)
+    for S in (3, 15, 16, 17, 63, 64, 65, 130, 257, 520):
+        q = torch.randn(2, Hq, Sq, D, device="cuda", generator=g).to(dtype)
+        k, v = (torch.randn(2, Hkv, S, D, device="cuda", generator=g).to(dtype) for _ in range(2))
+        kk, vv = k, v
+        if kind == "e5m2":
+            k, v = cuda_ops.quantize_kv_e5m2(k), cuda_ops.quantize_kv_e5m2(v)
+            kk, vv = cuda_ops.dequantize_kv_e5m2(k, dtype), cuda_ops.dequantize_kv_e5m2(v, dtype)
+        kd, vd = (t.double().repeat_interleave(Hq // Hkv, 1) for t in (kk, vv))
+        s = q.double() @ kd.transpose(-1, -2) / math.sqrt(D)
+        hidden = torch.arange(S, device="cuda")[None] > torch.arange(S - Sq, S, device="cuda")[:, None]
+        p = torch.softmax(s.masked_fill(hidden, float("-inf")), -1)
+        ref = p @ vd
+        # 32-bit sums and an approximate exponential (2^-20 of the weights, with scores up to a few dozen), then the rounding
+        bound = ref.abs() * u + (p @ vd.abs()) * 2.0 ** -17 + 1e-7
+        for n in (1, 2, 3, 8):
+            monkeypatch.setattr(cuda_ops, "attn_splits", lambda *a, n=n: n)
+            out = cuda_ops.sdpa_decode(q, k, v, None, 1.0 / math.sqrt(D), None, None)
+            torch.cuda.synchronize()
+            assert bool(((out.double() - ref).abs() <= bound).all()), (S, n)
+
+
+def test_splits_fit_the_gpu(monkeypatch):
+    from ipex_llm_b200.ops import cuda_ops
+    monkeypatch.delenv("IPEX_LLM_ATTN_STEPS", raising=False)
+    monkeypatch.delenv("IPEX_LLM_ATTN_MIN_CTAS", raising=False)
+    for B in (1, 3, 8, 32, 700):
+        for Hkv, rows in ((32, 1), (8, 8), (1, 71)):
+            for S in (1, 40, 1000, 100000):
+                n = cuda_ops.attn_splits(B, Hkv, S, rows, 128, False, torch.bfloat16)
+                per_sm = cuda_ops._attn_ctas_per_sm(128, rows, False, 1)
+                assert 1 <= n <= 128 and (n == 1 or n * B * Hkv * -(-rows // 16) <= 148 * per_sm and S // n >= 160)
