@@ -701,15 +701,29 @@ class DecoderEngine:
         cos = torch.cat([self.cos[:S], self.cos[:S]], dim=-1).unsqueeze(0)             # [1, S, R] fp32
         sin = torch.cat([self.sin[:S], self.sin[:S]], dim=-1).unsqueeze(0)
         scale = 1.0 / math.sqrt(D)
+        # rotation over whole heads and a cache of the engine's own: everything between qkv and attention in one pass
+        first = cache.layers[self.layers[0].layer_idx]
+        one_pass = self.rot_dim == D and D % 16 == 0 and D <= 256 and first._k.dtype in (torch.uint8, self.dtype) and \
+            first._k.stride(3) == 1 and first._k.stride() == first._v.stride()
         for L in self.layers:
             x = cuda_ops.rms_norm(h, L.ln1, self.eps)
             qkv = self._gemm(L.qkv, x).view(B, S, Hq + 2 * Hkv, D)
             q = qkv[:, :, :Hq].transpose(1, 2)                                          # [B, Hq, S, D] views
             k = qkv[:, :, Hq:Hq + Hkv].transpose(1, 2)
             v = qkv[:, :, Hq + Hkv:].transpose(1, 2)
-            q, k = cuda_ops.rotary_inplace(q, k, cos, sin)
-            cache.layers[L.layer_idx].update(k, v)
-            a = cuda_ops.sdpa_prefill(q, k, v, None, scale, None, None, causal=True)    # [B, Hq, S, D]
+            layer = cache.layers[L.layer_idx]
+            if one_pass:
+                tc = cuda_ops.attn_prefill_tcgen05_ok(q, k, v)
+                vt = cuda_ops.prompt_prep(qkv.view(T, -1), layer._k, layer._v, self.cos, self.sin, B, S, Hq, Hkv, D, tc)
+                layer.set_length(S)
+                if tc:
+                    a = cuda_ops.attn_prefill_tcgen05(q, k, v, scale, True, vt=vt)      # [B, Hq, S, D]
+                else:
+                    a = cuda_ops.sdpa_prefill(q, k, v, None, scale, None, None, causal=True)
+            else:
+                q, k = cuda_ops.rotary_inplace(q, k, cos, sin)
+                layer.update(k, v)
+                a = cuda_ops.sdpa_prefill(q, k, v, None, scale, None, None, causal=True)
             a = a.transpose(1, 2).reshape(T, Hq * D)
             h1 = self._gemm(L.o, a, residual=h)
             if L.moe is not None:

@@ -579,18 +579,36 @@ def attn_prefill_tcgen05_ok(q, k, v) -> bool:
     return _token_major(q) and _token_major(k)
 
 
+def prompt_prep(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, B: int,
+                S: int, Hq: int, Hkv: int, D: int, transpose_v: bool):
+    """What lies between the qkv product of whole prompts ``[B * S, (Hq + 2 Hkv) * D]`` and their attention, in one pass:
+    queries and keys rotated in place (halves of D; ``cos`` / ``sin`` fp32 ``[>= S, D / 2]``), keys and values into rows
+    ``0 .. S - 1`` of the caches ``[B, Hkv, cap, D]`` (qkv's type, or e5m2 bytes).  Returns V transposed ``[B, Hkv, D, S
+    rounded up to 8]`` with zeros past S for ``attn_prefill_tcgen05`` (None unless asked for)."""
+    s_pad = (S + 7) // 8 * 8
+    vt = torch.empty(B, Hkv, D, s_pad, dtype=qkv.dtype, device=qkv.device) if transpose_v else None
+    rc = cuda_lib().ipex_prompt_prep(ptr(qkv), ptr(cos), ptr(sin), ptr(k_cache), ptr(v_cache), ptr(vt), B, S, Hq, Hkv, D,
+                                     qkv.stride(0), k_cache.stride(0), k_cache.stride(1), k_cache.stride(2), s_pad,
+                                     int(k_cache.dtype == torch.uint8), _dt(qkv), current_stream())
+    api.check(rc, "prompt_prep")
+    return vt
+
+
 def attn_prefill_tcgen05(q, k, v, scale: float, causal: bool = True, softcap: float = 0.0, window: int = 0,
-                         kv_lo: torch.Tensor = None) -> torch.Tensor:
+                         kv_lo: torch.Tensor = None, vt: torch.Tensor = None) -> torch.Tensor:
     """Prompt attention (Sq == Skv) on the tcgen05 kernel.  ``q [B, Hq, S, D]`` and ``k [B, Hkv, S, D]`` are
     token-major views (see ``_token_major``), already rotated; ``v`` any layout.  Returns ``[B, Hq, S, D]`` as a
     view of a ``[B, S, Hq, D]`` buffer, so the ``transpose(1, 2).reshape(T, Hq * D)`` that feeds the output
     projection is free.  ``softcap`` (Gemma-2 tanh cap of the scaled scores), ``window`` (sliding window) and
-    ``kv_lo`` (int32 ``[B]``: first real token of each left-padded row) are applied inside the kernel."""
+    ``kv_lo`` (int32 ``[B]``: first real token of each left-padded row) are applied inside the kernel.  ``vt``: v
+    transposed already (``prompt_prep``)."""
     lib = cuda_lib()
     B, Hq, S, D = q.shape
     Hkv = k.shape[1]
     s_pad = (S + 7) // 8 * 8
-    if _token_major(v) and B * Hkv <= 65535 and hasattr(lib, "ipex_attn_transpose_v"):
+    if vt is not None:
+        pass
+    elif _token_major(v) and B * Hkv <= 65535 and hasattr(lib, "ipex_attn_transpose_v"):
         # tiled transpose kernel (a strided torch copy of this shape runs at a fraction of the memory rate and
         # cost as much as the attention itself)
         vt = torch.empty(B, Hkv, D, s_pad, dtype=q.dtype, device=q.device)
