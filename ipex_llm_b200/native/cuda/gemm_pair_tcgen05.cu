@@ -51,6 +51,7 @@ struct PairArgs {
   int m_tiles, n_tiles;   // token tiles of BT, weight tiles of 256 rows
   int act;
   int* err;
+  const int* m_range;     // device: (first row, rows) of x and out that this launch covers, or null for all M
 };
 
 template <int WF> struct PairFam {
@@ -274,9 +275,16 @@ __device__ __forceinline__ void expand_role(const PairArgs& a, uint8_t* sA, uint
 
 template <typename T, int BT, int WF>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairFam<WF>::threads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const PairArgs a) {
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, PairArgs a) {
   using C = PairCfg<BT>;
   constexpr bool kDense = PairFam<WF>::dense;
+  int row0 = 0;
+  if (!kDense && a.m_range != nullptr) {
+    row0 = a.m_range[0];
+    a.M = a.m_range[1];
+    a.m_tiles = (a.M + BT - 1) / BT;
+    a.out = reinterpret_cast<T*>(a.out) + (int64_t)row0 * a.ldo;
+  }
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
@@ -343,7 +351,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           if (rank == 0) mbar_expect_tx(&full[s], 2 * (kDense ? C::kStageBytes : C::kBBytes));
           if constexpr (kDense)
             tma_load_2d_pair(sA + s * C::kABytes, &tm_w, kb * kBK, (nb * 2 + (int)rank) * kBM, full0 + s * 8);
-          tma_load_2d_pair(sB + s * C::kBBytes, &tm_x, kb * kBK, mb * BT + (int)rank * (BT / 2), full0 + s * 8);
+          tma_load_2d_pair(sB + s * C::kBBytes, &tm_x, kb * kBK, row0 + mb * BT + (int)rank * (BT / 2), full0 + s * 8);
         }
         if (++s == C::kStages) { s = 0; ph ^= 1; }
       }
@@ -500,11 +508,10 @@ cudaError_t dispatch_wf(int wf, int bt, const CUtensorMap& tw, const CUtensorMap
 
 }  // namespace
 
-// The product of ipex_gemm_lowbit_tcgen05 (packed `w`) or ipex_gemm_tcgen05_act (dense `w`, row stride ldw) on SM pairs.
-// `bt`: token tile, 128 or 256.  Arguments as checked there.
-IPEX_API int ipex_gemm_pair_tcgen05(const void* x, const void* w, void* out, const void* bias, const void* residual,
-                                    const float* lut, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo,
-                                    int64_t ldr, int wf, int act, int dtype, int bt, int* err, void* stream) {
+// Rows [m_range[0], m_range[0] + m_range[1]) (device memory) of x [M, K] when m_range is given, with a grid for m_upper rows.
+static int pair_entry(const void* x, const void* w, void* out, const void* bias, const void* residual, const float* lut,
+                      const int* m_range, int m_upper, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo,
+                      int64_t ldr, int wf, int act, int dtype, int bt, int* err, void* stream) {
   const bool dense = wf == WF_F16 || wf == WF_BF16;
   if (M < 1 || N < 1 || K < 1 || (ldx % 8) != 0 || (bt != 128 && bt != 256)) return (int)cudaErrorInvalidValue;
   if (reinterpret_cast<uintptr_t>(x) & 15) return (int)cudaErrorInvalidValue;
@@ -522,8 +529,9 @@ IPEX_API int ipex_gemm_pair_tcgen05(const void* x, const void* w, void* out, con
   a.w = reinterpret_cast<const uint8_t*>(w); a.lut = lut;
   a.out = out; a.bias = bias; a.residual = residual; a.ldo = ldo; a.ldr = ldr;
   a.Np = ceil_to_i64(N, 16); a.Kp = ceil_to_i64(K, 128);
-  a.M = M; a.N = N; a.K = K;
-  a.m_tiles = (M + bt - 1) / bt;
+  a.M = m_upper; a.N = N; a.K = K;
+  a.m_range = m_range;
+  a.m_tiles = (m_upper + bt - 1) / bt;
   a.n_tiles = (N + 2 * kBM - 1) / (2 * kBM);
   a.act = act;
   a.err = err;
@@ -533,4 +541,20 @@ IPEX_API int ipex_gemm_pair_tcgen05(const void* x, const void* w, void* out, con
   cudaStream_t st = (cudaStream_t)stream;
   return (int)(dtype == DT_F16 ? dispatch_wf<__half>(wf, bt, tw, tx, a, sms, st)
                                : dispatch_wf<__nv_bfloat16>(wf, bt, tw, tx, a, sms, st));
+}
+
+// The product of ipex_gemm_lowbit_tcgen05 (packed `w`) or ipex_gemm_tcgen05_act (dense `w`, row stride ldw) on SM pairs.
+// `bt`: token tile, 128 or 256.  Arguments as checked there.
+IPEX_API int ipex_gemm_pair_tcgen05(const void* x, const void* w, void* out, const void* bias, const void* residual,
+                                    const float* lut, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo,
+                                    int64_t ldr, int wf, int act, int dtype, int bt, int* err, void* stream) {
+  return pair_entry(x, w, out, bias, residual, lut, nullptr, M, M, N, K, ldx, ldw, ldo, ldr, wf, act, dtype, bt, err, stream);
+}
+
+// One expert's product of ipex_gemm_lowbit_tcgen05_grouped on SM pairs.
+IPEX_API int ipex_gemm_pair_tcgen05_grouped(const void* x, const void* w, void* out, const float* lut, const int* m_range,
+                                            int M_total, int m_upper, int N, int K, int64_t ldx, int64_t ldo, int wf, int act,
+                                            int dtype, int bt, int* err, void* stream) {
+  return pair_entry(x, w, out, nullptr, nullptr, lut, m_range, m_upper, M_total, N, K, ldx, 0, ldo, 0, wf, act, dtype, bt, err,
+                    stream);
 }

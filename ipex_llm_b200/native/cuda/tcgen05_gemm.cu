@@ -601,6 +601,9 @@ IPEX_API int ipex_gemm_pair_tcgen05(const void* x, const void* w, void* out, con
                                     const float* lut, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo,
                                     int64_t ldr, int wf, int act, int dtype, int bt, int* err, void* stream);
 
+IPEX_API int ipex_gemm_pair_tcgen05_grouped(const void* x, const void* w, void* out, const float* lut, const int* m_range,
+                                            int M_total, int m_upper, int N, int K, int64_t ldx, int64_t ldo, int wf, int act,
+                                            int dtype, int bt, int* err, void* stream);
 // gemm_few_tcgen05.cu: packed weights with up to 64 rows.
 IPEX_API int ipex_gemm_few_tcgen05(const void* x, const void* w, void* out, const void* bias, const void* residual,
                                    const float* lut, int M, int N, int K, int64_t ldx, int64_t ldo, int64_t ldr, int wf,
@@ -711,6 +714,10 @@ IPEX_API int ipex_gemm_lowbit_tcgen05_grouped(const void* x, const void* w, void
   if (act != 0 && (N % 32) != 0) return (int)cudaErrorInvalidValue;
   if (wf == WF_LUT4 && lut == nullptr) return (int)cudaErrorInvalidValue;
   if (bt != 32 && bt != 64 && bt != 128 && bt != 256) return (int)cudaErrorInvalidValue;
+  if (wf < WF_SYM_INT4 || wf > WF_INT8) return (int)cudaErrorInvalidValue;
+  if (bt >= 128 && (reinterpret_cast<uintptr_t>(w) & 31) == 0)   // as for one matrix: the pair wins at every such size
+    return ipex_gemm_pair_tcgen05_grouped(x, w, out, lut, m_range, M_total, m_upper, N, K, ldx, ldo, wf, act, dtype, bt, err,
+                                          stream);
   const CUtensorMapDataType tdt = dtype == DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUtensorMap tx;
   if (!tc5::encode_2d_sw128(&tx, tdt, x, (uint64_t)K, (uint64_t)M_total, (uint64_t)ldx * 2, kBK, bt)) return -1;
