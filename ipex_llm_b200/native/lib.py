@@ -126,5 +126,6 @@ def ptr(t) -> ctypes.c_void_p:
 
 
 def current_stream() -> ctypes.c_void_p:
+    """Handle of the current CUDA stream of the current device (no stream object is made for it)."""
     import torch
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))

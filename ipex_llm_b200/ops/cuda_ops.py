@@ -34,11 +34,18 @@ _lut_cache = {}
 _USE_PDL = os.environ.get("IPEX_LLM_PDL", "1") != "0"
 _GEMV_IMPL = os.environ.get("IPEX_LLM_GEMV", "stream")   # stream | tma | v1
 _err_flags = {}
+_err_flag_of = {}      # the same by torch.device: the look-up of every launch
 
 
 def error_flag(device) -> torch.Tensor:
     """Device int the kernels with bounded waits set when a wait expires (0 = healthy)."""
-    key = str(device)
+    flag = _err_flag_of.get(device)
+    if flag is None:
+        flag = _err_flag_of[device] = _make_error_flag(str(device), device)
+    return flag
+
+
+def _make_error_flag(key: str, device) -> torch.Tensor:
     if key not in _err_flags:
         _err_flags[key] = torch.zeros(4, dtype=torch.int32, device=device)
         tune = os.environ.get("IPEX_LLM_GEMV_TUNE")  # "ctas_per_sm,budget_kb,chunks_per_stage"
