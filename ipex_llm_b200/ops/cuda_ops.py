@@ -276,6 +276,8 @@ def dequantize_device(w_data: torch.Tensor, shape, qtype: int, dtype=torch.float
     lib = cuda_lib()
     out = torch.empty((N, K), dtype=dtype, device=w_data.device)
     if is_tiled(qtype):
+        if w_data.data_ptr() % 16:
+            w_data = w_data.clone()          # a slice in the middle of other bytes: the kernel reads 16 at a time
         rc = lib.ipex_dequantize_tiles(ptr(w_data), ptr(out), N, K, K, QTYPE_TO_WF[qtype],
                                        ptr(lut_for(qtype, w_data.device)), api.dtype_code(dtype), current_stream())
         api.check(rc, "dequantize_tiles")

@@ -39,6 +39,8 @@ def quantize_to_device_layout(w: torch.Tensor, qtype: int, out: torch.Tensor = N
     nbytes = device_nbytes(rows, cols, qtype)
     if out is None:
         out = torch.empty(nbytes, dtype=torch.uint8, device=w.device)       # the kernel writes every byte, padding too
+    if out.data_ptr() % 16:                  # a slice in the middle of other bytes: the kernel writes 16 at a time
+        return out.copy_(quantize_to_device_layout(w, qtype).view_as(out))
     wf, lut_kind = _GPU_QTYPES[qtype]
     rc = lib.ipex_quantize_to_tiles(ptr(w2), ptr(out), rows, cols, w2.stride(0), wf, lut_kind,
                                     api.dtype_code(w2.dtype), current_stream())

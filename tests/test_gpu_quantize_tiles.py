@@ -41,3 +41,18 @@ def test_pack_and_expand(name, shape, dtype):
         assert torch.equal(back, host)
     for half in (torch.float16, torch.bfloat16):
         assert torch.equal(dequantize_device(packed, (N, K), q, half).cpu(), back.to(half))
+
+
+def test_slices_between_other_bytes():
+    """Packed bytes that begin anywhere in a larger buffer."""
+    from ipex_llm_b200.ops.cuda_ops import dequantize_device
+    from ipex_llm_b200.ops.cuda_quant import quantize_to_device_layout
+    from ipex_llm_b200.quant import qtypes as qt
+    w = torch.randn(40, 256, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).half()
+    packed = quantize_to_device_layout(w, qt.SYM_INT4)
+    buf = torch.full((packed.numel() + 8,), 0xA5, dtype=torch.uint8, device="cuda")
+    part = buf[4:4 + packed.numel()]
+    assert torch.equal(quantize_to_device_layout(w, qt.SYM_INT4, out=part), packed) and torch.equal(part, packed)
+    assert bool((buf[:4] == 0xA5).all()) and bool((buf[-4:] == 0xA5).all())
+    dense = dequantize_device(packed, (40, 256), qt.SYM_INT4, torch.float16)
+    assert torch.equal(dequantize_device(part, (40, 256), qt.SYM_INT4, torch.float16), dense)
