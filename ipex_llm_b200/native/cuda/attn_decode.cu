@@ -302,7 +302,22 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
     }
   };
 
-  for (int base = t0 + tsub * 4; base < t1; base += kPF * stride) {
+  // Keys in [seen_lo, seen_hi) are seen by every row of the warp: all of a decode step's, unless there is a window or several
+  // queries.  A batch outside has to ask for each row, and a hidden key's value takes no part, not even with weight zero: it
+  // may hold anything (0 * inf).  Two bodies, because the questions in the loop cost more than the second body does: 32
+  // sequences x 32 heads of 2048 tokens in fp16 197 us with them and 184 without; 8 query heads to each of 8 kv heads, 2048
+  // e5m2 tokens in 12 splits 36.6 and 33.0.
+  int seen_lo = 0, seen_hi = t1;
+#pragma unroll
+  for (int r = 0; r < RW; r++) {
+    if (causal && qpos[r] >= 0) {
+      const int limit = causal_base + qpos[r] + 1;
+      seen_hi = min(seen_hi, limit);
+      if (a.window > 0) seen_lo = max(seen_lo, limit - a.window);
+    }
+  }
+  auto batch = [&](int base, auto seen_by_all) {
+    constexpr bool kAll = decltype(seen_by_all)::value;
     float sc[kPF][RW];
 #pragma unroll
     for (int i = 0; i < kPF; i++) {
@@ -331,6 +346,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
 #pragma unroll
         for (int r = 0; r < RW; r++) sc[i][r] += __shfl_xor_sync(0xffffffffu, sc[i][r], o);
     float corr[RW];
+    uint32_t hidden = 0;                                 // bit i * RW + r: the row does not see the step's key
 #pragma unroll
     for (int r = 0; r < RW; r++) {
       float mn = m[r];
@@ -339,10 +355,13 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
         const int pos = base + i * stride + tg;
         float s = sc[i][r];
         if (cap > 0.f) s = cap * tanhf(s * inv_cap_scaled);
-        bool ok = pos < t1 && qpos[r] >= 0;
-        if (ok && causal) {
-          const int limit = causal_base + qpos[r] + 1;
-          ok = pos < limit && (a.window <= 0 || pos >= limit - a.window);
+        bool ok = pos < t1;
+        if constexpr (!kAll) {
+          if (causal) {
+            const int limit = causal_base + qpos[r] + 1;
+            ok = ok && pos < limit && (a.window <= 0 || pos >= limit - a.window);
+          }
+          if (!ok) hidden |= 1u << (i * RW + r);
         }
         sc[i][r] = ok ? s : -INFINITY;
         mn = fmaxf(mn, sc[i][r]);
@@ -369,8 +388,13 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
 #pragma unroll
       for (int r = 0; r < RW; r++)
 #pragma unroll
-        for (int d = 0; d < DPL; d++) acc[r][d] += sc[i][r] * vf[d];
+        for (int d = 0; d < DPL; d++)
+          if (kAll || ((hidden >> (i * RW + r)) & 1) == 0) acc[r][d] += sc[i][r] * vf[d];
     }
+  };
+  for (int base = t0 + tsub * 4; base < t1; base += kPF * stride) {
+    if (base >= seen_lo && min(t1, base + kPF * stride) <= seen_hi) batch(base, std::true_type());
+    else batch(base, std::false_type());
   }
   // ---- new tokens (mode A, last split) from shared memory ----
   if (modeA && last_split) {

@@ -37,6 +37,34 @@ def test_walk(kind, D, heads, monkeypatch):
             assert bool(((out.double() - ref).abs() <= bound).all()), (S, n)
 
 
+@pytest.mark.parametrize("heads", [(4, 4, 1), (8, 2, 1), (4, 2, 3), (16, 1, 1)])     # one, four, six and sixteen rows a head
+@pytest.mark.parametrize("kind", ["half", "e5m2"])
+def test_hidden_values_do_not_count(kind, heads, monkeypatch):
+    """A value row that a query does not see (left of its window, or of a later query's token) may hold anything."""
+    from ipex_llm_b200.ops import cuda_ops
+    Hq, Hkv, Sq = heads
+    D, window = 128, 50
+    g = torch.Generator(device="cuda").manual_seed(Hq + Sq)
+    for S in (64, 65, 130, 300):
+        q = torch.randn(1, Hq, Sq, D, device="cuda", generator=g).half()
+        k, v = (torch.randn(1, Hkv, S, D, device="cuda", generator=g).half() for _ in range(2))
+        code = cuda_ops.quantize_kv_e5m2 if kind == "e5m2" else (lambda t: t)
+        k, v = code(k), code(v)
+        bad = v.clone()
+        unseen = S - Sq - window + 1                       # the first query sees the `window` positions from here on
+        inf = 0x7C if kind == "e5m2" else float("inf")
+        bad[:, :, :unseen] = inf
+        if Sq > 1:
+            bad[:, :, S - 1] = inf                         # only the last query sees the last position
+        for n in (1, 3):
+            monkeypatch.setattr(cuda_ops, "attn_splits", lambda *a, n=n: n)
+            ref = cuda_ops.sdpa_decode(q, k, v, None, 1.0 / math.sqrt(D), None, window)
+            out = cuda_ops.sdpa_decode(q, k, bad, None, 1.0 / math.sqrt(D), None, window)
+            torch.cuda.synchronize()
+            rows = slice(0, max(1, Sq - 1))
+            assert torch.equal(out[:, :, rows], ref[:, :, rows]), (S, n)
+
+
 def test_splits_fit_the_gpu(monkeypatch):
     from ipex_llm_b200.ops import cuda_ops
     monkeypatch.delenv("IPEX_LLM_ATTN_STEPS", raising=False)
