@@ -698,13 +698,10 @@ class DecoderEngine:
             h = hidden.reshape(B * S, self.H).to(self.dtype)
         T, H, D = B * S, self.H, self.hd
         Hq, Hkv = self.n_heads, self.n_kv
-        cos = torch.cat([self.cos[:S], self.cos[:S]], dim=-1).unsqueeze(0)             # [1, S, R] fp32
-        sin = torch.cat([self.sin[:S], self.sin[:S]], dim=-1).unsqueeze(0)
         scale = 1.0 / math.sqrt(D)
-        # rotation over whole heads and a cache of the engine's own: everything between qkv and attention in one pass
-        first = cache.layers[self.layers[0].layer_idx]
-        one_pass = self.rot_dim == D and D % 16 == 0 and D <= 256 and first._k.dtype in (torch.uint8, self.dtype) and \
-            first._k.stride(3) == 1 and first._k.stride() == first._v.stride()
+        # rotation over whole heads: everything between qkv and attention in one pass, where the layer's cache holds the prompt
+        # as it is (its rows may have been selected, or its storage replaced, since the last one)
+        whole = self.rot_dim == D and D % 16 == 0 and D <= 256
         for L in self.layers:
             x = cuda_ops.rms_norm(h, L.ln1, self.eps)
             qkv = self._gemm(L.qkv, x).view(B, S, Hq + 2 * Hkv, D)
@@ -712,7 +709,7 @@ class DecoderEngine:
             k = qkv[:, :, Hq:Hq + Hkv].transpose(1, 2)
             v = qkv[:, :, Hq + Hkv:].transpose(1, 2)
             layer = cache.layers[L.layer_idx]
-            if one_pass:
+            if whole and cuda_ops.prompt_prep_fits(layer._k, layer._v, self.cos, self.sin, self.dtype, B, S, Hkv, D):
                 tc = cuda_ops.attn_prefill_tcgen05_ok(q, k, v)
                 vt = cuda_ops.prompt_prep(qkv.view(T, -1), layer._k, layer._v, self.cos, self.sin, B, S, Hq, Hkv, D, tc)
                 layer.set_length(S)
@@ -721,6 +718,7 @@ class DecoderEngine:
                 else:
                     a = cuda_ops.sdpa_prefill(q, k, v, None, scale, None, None, causal=True)
             else:
+                cos, sin = (torch.cat([t[:S], t[:S]], dim=-1).unsqueeze(0) for t in (self.cos, self.sin))    # [1, S, R] fp32
                 q, k = cuda_ops.rotary_inplace(q, k, cos, sin)
                 layer.update(k, v)
                 a = cuda_ops.sdpa_prefill(q, k, v, None, scale, None, None, causal=True)

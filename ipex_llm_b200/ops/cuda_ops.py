@@ -588,12 +588,32 @@ def attn_prefill_tcgen05_ok(q, k, v) -> bool:
     return _token_major(q) and _token_major(k)
 
 
+def prompt_prep_fits(k_cache, v_cache, cos: torch.Tensor, sin: torch.Tensor, dtype: torch.dtype, B: int, S: int, Hkv: int,
+                     D: int) -> bool:
+    """Whether ``prompt_prep`` may write the first S rows of these caches for B sequences: it goes by their strides alone."""
+    if k_cache is None or v_cache is None or k_cache.shape != v_cache.shape or k_cache.stride() != v_cache.stride() or \
+            k_cache.dtype != v_cache.dtype or k_cache.dtype not in (torch.uint8, dtype):
+        return False
+    if k_cache.dim() != 4 or k_cache.shape[0] != B or k_cache.shape[1] != Hkv or k_cache.shape[2] < S or k_cache.shape[3] != D:
+        return False
+    if k_cache.stride(3) != 1 or any(n % 8 for n in k_cache.stride()[:3]) or \
+            any(t.data_ptr() % (8 * t.element_size()) for t in (k_cache, v_cache)):
+        return False
+    return all(t.dtype == torch.float32 and t.is_contiguous() and t.dim() == 2 and t.shape[0] >= S and t.shape[1] == D // 2
+               for t in (cos, sin))
+
+
 def prompt_prep(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, B: int,
                 S: int, Hq: int, Hkv: int, D: int, transpose_v: bool):
     """What lies between the qkv product of whole prompts ``[B * S, (Hq + 2 Hkv) * D]`` and their attention, in one pass:
     queries and keys rotated in place (halves of D; ``cos`` / ``sin`` fp32 ``[>= S, D / 2]``), keys and values into rows
     ``0 .. S - 1`` of the caches ``[B, Hkv, cap, D]`` (qkv's type, or e5m2 bytes).  Returns V transposed ``[B, Hkv, D, S
     rounded up to 8]`` with zeros past S for ``attn_prefill_tcgen05`` (None unless asked for)."""
+    if not prompt_prep_fits(k_cache, v_cache, cos, sin, qkv.dtype, B, S, Hkv, D) or qkv.dim() != 2 or qkv.stride(1) != 1 or \
+            qkv.shape[0] != B * S or qkv.shape[1] < (Hq + 2 * Hkv) * D:
+        raise ValueError("prompt_prep: %s rows of qkv, caches %s / %s and angles %s do not fit %d x %d tokens of %d + 2 x %d "
+                         "heads of %d" % (tuple(qkv.shape), tuple(k_cache.shape), tuple(v_cache.shape), tuple(cos.shape), B, S,
+                                          Hq, Hkv, D))
     s_pad = (S + 7) // 8 * 8
     vt = torch.empty(B, Hkv, D, s_pad, dtype=qkv.dtype, device=qkv.device) if transpose_v else None
     rc = cuda_lib().ipex_prompt_prep(ptr(qkv), ptr(cos), ptr(sin), ptr(k_cache), ptr(v_cache), ptr(vt), B, S, Hq, Hkv, D,
