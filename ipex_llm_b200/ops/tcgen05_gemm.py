@@ -114,12 +114,21 @@ def gemm_few(x: torch.Tensor, w_data: torch.Tensor, N: int, K: int, out: torch.T
              bias: torch.Tensor = None, residual: torch.Tensor = None, act: int = 0, pairs: bool = False,
              pdl: bool = False) -> bool:
     """``x @ dequant(w).T`` for few rows into ``out`` (see native/cuda/gemm_few_tcgen05.cu); ``pairs``: ``x`` holds value and
-    remainder of every token in turn (``cuda_ops.rms_norm_pairs``).  False when the operands do not suit the kernel."""
-    lib = cuda_lib()
-    M = out.shape[0]
-    if x.shape[0] > FEW_MAX_ROWS or x.stride(1) != 1 or x.stride(0) % 8 != 0 or x.data_ptr() % 16 != 0 or \
-            w_data.data_ptr() % 32 != 0 or (residual is not None and residual.stride(1) != 1):
+    remainder of every token in turn (``cuda_ops.rms_norm_pairs``).  False, and nothing is launched, when the operands do not
+    suit the kernel."""
+    M, n_out = out.shape[0], N // 2 if act else N
+    if x.dim() != 2 or x.shape[0] != (2 * M if pairs else M) or x.shape[0] > FEW_MAX_ROWS or x.shape[1] < K or \
+            x.stride(1) != 1 or x.stride(0) % 8 != 0 or x.data_ptr() % 16 != 0 or w_data.data_ptr() % 32 != 0:
         return False
+    if x.dtype not in (torch.float16, torch.bfloat16) or out.dtype != x.dtype or out.dim() != 2 or out.shape[1] < n_out or \
+            out.stride(1) != 1:
+        return False
+    if bias is not None and (bias.dtype != x.dtype or bias.dim() != 1 or bias.shape[0] < N or bias.stride(0) != 1):
+        return False
+    if residual is not None and (act or residual.dtype != x.dtype or residual.dim() != 2 or residual.shape[0] < M or
+                                 residual.shape[1] < n_out or residual.stride(1) != 1):
+        return False
+    lib = cuda_lib()
     rc = lib.ipex_gemm_few_tcgen05(ptr(x), ptr(w_data), ptr(out), ptr(bias), ptr(residual), ptr(lut), M, N, K, x.stride(0),
                                    out.stride(0), residual.stride(0) if residual is not None else 0, wf, int(act), int(pairs),
                                    api.dtype_code(x.dtype), int(pdl), ptr(_err(x.device)), current_stream())

@@ -1,0 +1,53 @@
+"""What the product for few rows refuses: it builds a tensor map of ``x``, and writes ``out``, from the sizes it is given."""
+import pytest
+import torch
+
+M, N, K = 5, 32, 128
+
+
+def _operands(pairs):
+    f16 = dict(dtype=torch.float16)
+    return dict(x=torch.zeros(2 * M if pairs else M, K, **f16), w_data=torch.zeros(4096 + 32, dtype=torch.uint8),
+                out=torch.zeros(M, N, **f16), bias=torch.zeros(N, **f16), residual=torch.zeros(M, N, **f16))
+
+
+BAD = {
+    "fewer rows": lambda o: o.update(x=o["x"][:-1]),
+    "more rows": lambda o: o.update(out=o["out"][:-1], residual=o["residual"][:-1]),
+    "shorter rows": lambda o: o.update(x=o["x"][:, :K - 8]),
+    "rows with gaps": lambda o: o.update(x=torch.zeros(o["x"].shape[0], 2 * K, dtype=torch.float16)[:, ::2]),
+    "rows of an odd stride": lambda o: o.update(x=torch.zeros(o["x"].shape[0], K + 4, dtype=torch.float16)[:, :K]),
+    "rows that begin at 8 bytes": lambda o: o.update(x=torch.zeros(o["x"].shape[0], K + 8, dtype=torch.float16)[:, 4:K + 4]),
+    "rows in 32 bits": lambda o: {k: o.update({k: o[k].float()}) for k in ("x", "out", "bias", "residual")},
+    "an output in 32 bits": lambda o: o.update(out=o["out"].float()),
+    "an output with gaps": lambda o: o.update(out=torch.zeros(M, 2 * N, dtype=torch.float16)[:, ::2]),
+    "an output that is too narrow": lambda o: o.update(out=o["out"][:, :N - 1]),
+    "a weight that begins at 16 bytes": lambda o: o.update(
+        w_data=o["w_data"][(16 - o["w_data"].data_ptr()) % 32:]),
+    "a bias that is too short": lambda o: o.update(bias=o["bias"][:-1]),
+    "a bias of another type": lambda o: o.update(bias=o["bias"].float()),
+    "a bias with gaps": lambda o: o.update(bias=torch.zeros(2 * N, dtype=torch.float16)[::2]),
+    "a residual of fewer rows": lambda o: o.update(residual=o["residual"][:-1]),
+    "a residual that is too narrow": lambda o: o.update(residual=o["residual"][:, :-1]),
+    "a residual of another type": lambda o: o.update(residual=o["residual"].bfloat16()),
+}
+
+
+@pytest.mark.parametrize("pairs", [False, True])
+@pytest.mark.parametrize("what", sorted(BAD))
+def test_refused(what, pairs):
+    from ipex_llm_b200.native import cuda_api as api
+    from ipex_llm_b200.ops import tcgen05_gemm
+    o = _operands(pairs)
+    o["w_data"] = o["w_data"][-o["w_data"].data_ptr() % 32:]
+    BAD[what](o)
+    assert tcgen05_gemm.gemm_few(o["x"], o["w_data"], N, K, o["out"], api.WF_SYM_INT4, bias=o["bias"], residual=o["residual"],
+                                 pairs=pairs) is False
+
+
+def test_pairs_need_two_rows_for_each_token():
+    from ipex_llm_b200.native import cuda_api as api
+    from ipex_llm_b200.ops import tcgen05_gemm
+    o = _operands(False)
+    o["w_data"] = o["w_data"][-o["w_data"].data_ptr() % 32:]
+    assert tcgen05_gemm.gemm_few(o["x"], o["w_data"], N, K, o["out"], api.WF_SYM_INT4, pairs=True) is False
