@@ -324,8 +324,10 @@ def rms_norm_pairs(x: torch.Tensor, weight: torch.Tensor, eps: float, offset: fl
     """RMSNorm of ``x [rows, H]`` in 32 bits, as ``[2 * rows, H]`` of x's type: every row's rounded values, then what the
     rounding left over (together twice the type's precision)."""
     rows, H = x.shape
+    xc = x.contiguous()
+    w = weight if weight.dtype == xc.dtype else weight.to(xc.dtype)
     out = torch.empty((2 * rows, H), dtype=x.dtype, device=x.device)
-    rc = cuda_lib().ipex_rms_norm_pairs(ptr(x), ptr(weight), ptr(out), rows, H, eps, offset, _dt(x), int(pdl and _USE_PDL),
+    rc = cuda_lib().ipex_rms_norm_pairs(ptr(xc), ptr(w), ptr(out), rows, H, eps, offset, _dt(x), int(pdl and _USE_PDL),
                                         current_stream())
     api.check(rc, "rms_norm_pairs")
     return out

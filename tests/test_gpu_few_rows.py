@@ -92,6 +92,21 @@ def test_rms_norm_rows(H, dtype):
     assert bool(((one - ref).abs() <= ref.abs() * (2.5 * U[dtype]) + 1e-7).all())    # value and product are rounded
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_norm_pairs_of_any_rows(dtype):
+    """Rows that are not packed one after another, and a weight of another type."""
+    from ipex_llm_b200.ops import cuda_ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(5, 512, device="cuda", generator=g).to(dtype)[:, :256]
+    w = 1 + 0.1 * torch.randn(256, device="cuda", generator=g)
+    for weight in (w.to(dtype), w):
+        pair = cuda_ops.rms_norm_pairs(x, weight, 1e-5)
+        assert torch.equal(pair, cuda_ops.rms_norm_pairs(x.contiguous(), weight.to(dtype), 1e-5))
+        ref = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * weight.to(dtype).double()
+        err = (pair.view(5, 2, 256).double().sum(1) - ref).abs()
+        assert bool((err <= ref.abs() * (U[dtype] ** 2 * 2 + 2.0 ** -20) + 2.0 ** -24).all())
+
+
 @pytest.mark.parametrize("batch", [9, 20, 32])
 def test_decode_steps_of_a_batch(batch):
     """Steps of a batch against the same sequences decoded eight at a time."""
