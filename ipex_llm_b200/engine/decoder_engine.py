@@ -587,14 +587,14 @@ class DecoderEngine:
 
     def _few_decode_ok(self) -> bool:
         """Decode steps of nine to 24 sequences on the product for few rows: formats it multiplies by without rounding them,
-        no experts, one GPU."""
+        weights that begin at 32 bytes (the GEMVs take 16), no experts, one GPU."""
         from ..ops import tcgen05_gemm
         ok = self.__dict__.get("_few_ok")
         if ok is None:
             ws = [w for L in self.layers for w in (L.qkv, L.o, L.gate_up, L.down)] + ([self.lm_head] if self.last_stage else [])
             ok = self._gemm_decode_ok() and not self.has_moe and self.H % 8 == 0 and self.H <= 16384 and \
                 all(w is not None and w.K % 128 == 0 and w.N % 16 == 0 and w.wf not in (api.WF_F16, api.WF_BF16) and
-                    tcgen05_gemm.few_exact(w.wf, self.dtype, 1) for w in ws)
+                    w.data.data_ptr() % 32 == 0 and tcgen05_gemm.few_exact(w.wf, self.dtype, 1) for w in ws)
             self._few_ok = ok
         return ok
 

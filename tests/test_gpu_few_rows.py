@@ -19,6 +19,13 @@ def _weights(name, N, K, dtype, g):
     return q, packed, cuda_ops.dequantize_device(packed, (N, K), q, torch.float32).double()
 
 
+def _at_16_bytes(t):
+    """The same bytes at an address that is a multiple of 16 but not of 32."""
+    room = torch.empty(t.numel() + 16, dtype=t.dtype, device=t.device)
+    room[16:].copy_(t)
+    return room[16:]
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("name", ["sym_int4", "asym_int4", "nf4", "fp8_e4m3", "fp8_e5m2", "sym_int8"])
@@ -132,3 +139,25 @@ def test_decode_steps_of_a_batch(batch):
     parts = torch.cat([steps(ids[s:s + 8]) for s in range(0, batch, 8)], dim=1)
     # both round every activation to fp16 about thirty times on the way: 2^-11 each, and no more than a few of them add up
     assert float((whole - parts).norm() / parts.norm()) < 8 * 2.0 ** -11
+
+
+def test_batch_whose_weights_begin_at_16_bytes():
+    from transformers import LlamaConfig
+    from ipex_llm_b200.engine.decoder_engine import DecoderEngine
+    from ipex_llm_b200.transformers import AutoModelForCausalLM
+    cfg = LlamaConfig(hidden_size=512, intermediate_size=1408, num_hidden_layers=2, num_attention_heads=4,
+                      num_key_value_heads=4, vocab_size=1024, max_position_embeddings=512, tie_word_embeddings=False)
+    model = AutoModelForCausalLM.from_config(cfg, load_in_low_bit="sym_int4", device="cuda:0", torch_dtype=torch.float16)
+    ids = torch.randint(0, 1024, (9, 24), device="cuda", generator=torch.Generator(device="cuda").manual_seed(9))
+
+    def step(move):
+        eng = DecoderEngine(model, max_batch=9, max_len=256, kv_fp8=False)
+        if move:
+            eng.layers[1].down.data = _at_16_bytes(eng.layers[1].down.data)
+        eng.prefill(ids)
+        eng.tokens[:9] = ids[:, 0]
+        eng.decode_step(9)
+        return eng.logits[:9].double().clone()
+
+    want, got = step(False), step(True)
+    assert float((got - want).norm() / want.norm()) < 8 * 2.0 ** -11
