@@ -101,7 +101,9 @@ __global__ void __launch_bounds__(512) rms_rows_kernel(const T* __restrict__ x, 
       float f = DT<T>::to_f(e[j]) * rstd;
       if (!PAIRS) f = DT<T>::to_f(DT<T>::from_f(f));   // HF casts the normalised value before the weight multiply
       f *= g;
-      hi[j] = DT<T>::from_f(f);
+      float h = f;                                     // past fp16's range the largest number, and the rest is the remainder
+      if (PAIRS && std::is_same<T, __half>::value) h = f > 65504.f ? 65504.f : f < -65504.f ? -65504.f : f;
+      hi[j] = DT<T>::from_f(h);
       if (PAIRS) lo[j] = DT<T>::from_f(f - DT<T>::to_f(hi[j]));
     }
     uint4* to = reinterpret_cast<uint4*>(y + (size_t)blockIdx.x * (PAIRS ? 2 : 1) * H);

@@ -114,6 +114,20 @@ def test_norm_pairs_of_any_rows(dtype):
         assert bool((err <= ref.abs() * (U[dtype] ** 2 * 2 + 2.0 ** -20) + 2.0 ** -24).all())
 
 
+def test_norm_pairs_past_the_range_of_half():
+    """Value and remainder add up to what a single fp16 number could not hold."""
+    from ipex_llm_b200.ops import cuda_ops
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(3, 512, device="cuda", generator=g).half()
+    w = torch.full((512,), 30000.0, device="cuda").half()
+    ref = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    assert 65504 < float(ref.abs().max()) < 131008
+    pair = cuda_ops.rms_norm_pairs(x, w, 1e-5).view(3, 2, 512).double()
+    # the remainder of a value past the range is rounded to fp16 itself
+    assert bool(((pair.sum(1) - ref).abs() <= ref.abs() * (U[torch.float16] ** 2 * 2 + 2.0 ** -20) +
+                 (ref.abs() > 65504) * 65504 * U[torch.float16]).all())
+
+
 @pytest.mark.parametrize("batch", [9, 20, 32])
 def test_decode_steps_of_a_batch(batch):
     """Steps of a batch against the same sequences decoded eight at a time."""
