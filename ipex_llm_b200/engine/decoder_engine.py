@@ -195,7 +195,9 @@ class DecoderEngine:
         self._graphs = {}
         self._lib = cuda_lib()
         self._nsplit = None
-        self._kv_hint = None       # prompt length of the current generation (sizes the attention splits)
+        self._kv_hint = None       # prompt length of the current generation
+        # contexts [_kv_from, _kv_until] that the attention splits are sized for, and as many tokens as the cache can hold by now
+        self._kv_from = self._kv_until = self._kv_bound = 0
         self._mega = None          # whole-step kernel launcher, created on first use (False = not applicable)
 
     # ------------------------------------------------------------------------------------------------
@@ -322,13 +324,27 @@ class DecoderEngine:
             out.copy_(y)
         return out
 
-    def _pick_splits(self, B: int) -> int:
-        """KV splits of the decode attention, sized for the context this generation starts from (with 256 tokens to come)
-        rather than for the cache capacity: the kernel divides whatever length it finds by this count.  The count is part
-        of the captured graph, so graphs are kept per (batch, splits)."""
-        hint = self._kv_hint if self._kv_hint else self.max_len
-        return cuda_ops.attn_splits(B, self.n_kv, min(hint + 256, self.max_len), self.n_heads // self.n_kv, self.hd,
-                                    self.kv_fp8, self.dtype)
+    def _seat_context(self, n: int):
+        """Sizes the attention splits for contexts from ``n`` tokens on: half as many again, at least 64 and at most 512."""
+        self._kv_from = self._kv_bound = n
+        self._kv_until = n + min(512, max(64, n // 2))
+
+    def _pick_splits(self, B: int, new: int = 1) -> int:
+        """KV splits of the decode attention of a step that adds ``new`` tokens, sized for the middle of the contexts that
+        the generation is about to reach rather than for the cache capacity: the kernel divides whatever length it finds by
+        this count, so a long reply to a short prompt needs more of them as it grows (one sequence, 8 kv heads of 8 rows:
+        2048 tokens 64 us in the four splits that 32 tokens get, 37 in twelve).  The host counts the tokens it has sent;
+        when they may be past what the count was sized for, it reads how many there are, because callers go back (rejected
+        drafts, the same continuation again).  The count is part of the captured graph, so graphs are kept per (batch,
+        splits)."""
+        if self._kv_hint is None:
+            kv = self.max_len
+        else:
+            self._kv_bound += new
+            if self._kv_bound > self._kv_until and not torch.cuda.is_current_stream_capturing():
+                self._seat_context(int(self.past_len[:B].max()) + new)
+            kv = min((self._kv_from + self._kv_until) // 2, self.max_len)
+        return cuda_ops.attn_splits(B, self.n_kv, kv, self.n_heads // self.n_kv, self.hd, self.kv_fp8, self.dtype)
 
     def _attention(self, L: _Layer, B: int, Sq: int = 1):
         """Rope + cache append + attention for ``B`` sequences of ``Sq`` new tokens each; rows of the activation
@@ -410,7 +426,7 @@ class DecoderEngine:
             raise ValueError(f"verify_step scores 1..{min(8, self.max_batch)} tokens, got {S}")
         if self.layers[0].o.tp is not None:
             raise NotImplementedError("verify_step runs on a single GPU")
-        self._nsplit = self._pick_splits(1)
+        self._nsplit = self._pick_splits(1, S)
         if not use_graph or os.environ.get("IPEX_LLM_ENGINE_GRAPH", "1") == "0":
             self._verify_kernels(S)
             return
@@ -574,6 +590,7 @@ class DecoderEngine:
         logits = out.logits[:, -1, :]
         self.past_len[:B] = S
         self._kv_hint = S
+        self._seat_context(S)
         return logits
 
     # ------------------------------------------------------------------------------------------------
@@ -687,6 +704,7 @@ class DecoderEngine:
         out = self.model(past_key_values=cache, use_cache=True, **kw).logits
         self.past_len[:B] = S
         self._kv_hint = S
+        self._seat_context(S)
         return out[:, -1, :] if self.last_stage else out
 
     def _prefill_flat(self, input_ids: torch.Tensor, cache, hidden: torch.Tensor = None):
@@ -732,6 +750,7 @@ class DecoderEngine:
             h = self._gemm(L.down, act, residual=h1)
         self.past_len[:B] = S
         self._kv_hint = S
+        self._seat_context(S)
         if not self.last_stage:
             return h.view(B, S, H)
         last = h.view(B, S, H)[:, -1].contiguous()

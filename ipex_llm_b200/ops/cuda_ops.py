@@ -477,15 +477,20 @@ def attn_splits(B: int, Hkv: int, kv_len: int, rows: int, head_dim: int, fp8: bo
     length).  As many as the GPU holds CTAs of at once (a second wave doubles the launch: 8 sequences x 32 heads of 517
     tokens 17 us at 2 splits, 24 at 4), and no walk shorter than it takes to pay for handing its sums over: 160 tokens, or
     512 where the heads alone fill the GPU (8 x 517 tokens 15.9 us whole, 17.3 in two; 8 x 2048 49 and 39; one sequence of
-    1024 11.3 us at 8 splits, 12.3 at 11, 13.1 at 3).  ``pick_nsplit``'s rule, which knows the walk's length only, where its
-    switches ask for it."""
+    1024 11.3 us at 8 splits, 12.3 at 11, 13.1 at 3).  Handing over costs the same for two parts as for four, so a walk that
+    is split at all is split in four: 32 heads of 128 tokens 7.6 us whole, 9.5 in two, 9.3 in four, of 256 tokens 10.2, 10.7
+    and 9.6; 8 kv heads of 8 rows, whose warps divide the rows and walk all tokens, 64 tokens 16.2, 18.9 and 17.1, 128 tokens
+    21.0, 21.3 and 18.4.  ``pick_nsplit``'s rule, which knows the walk's length only, where its switches ask for it."""
     if "IPEX_LLM_ATTN_STEPS" in os.environ or "IPEX_LLM_ATTN_MIN_CTAS" in os.environ:
         return pick_nsplit(B, Hkv, kv_len, rows=rows)
     heads = B * Hkv * -(-max(1, rows) // 16)
     wave = 148 * _attn_ctas_per_sm(head_dim, max(1, rows), bool(fp8), api.dtype_code(dtype)) // heads
-    n = min(wave, kv_len // (512 if heads >= 148 else 160))
+    if heads >= 148:
+        n = kv_len // 512
+    else:
+        n = max(4, kv_len // 160) if kv_len >= (192 if rows <= 1 else 96) else 1
     # a captured step keeps its count: few different ones, so that prompts of similar length share a graph
-    return max(c for c in (1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128) if c <= max(1, n))
+    return max(c for c in (1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128) if c <= max(1, min(n, wave)))
 
 
 _attn_ws_retired = []
