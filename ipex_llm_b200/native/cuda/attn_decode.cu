@@ -110,7 +110,10 @@ struct RawKV {
   }
 };
 
-template <typename T, bool FP8, int D, int RW>
+// HIDES: some query may not see some cached key (a window, or several queries whose keys are in the cache already).  Only then
+// a row asks for each key: the questions cost 5 - 12 % of a walk (32 sequences x 32 heads of 2048 fp16 tokens 197 us with
+// them and 184 without; 8 query heads to each of 8 kv heads, 2048 e5m2 tokens in 12 splits 36.6 and 33.0).
+template <typename T, bool FP8, int D, int RW, bool HIDES>
 __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
   constexpr int DPL = D / 8;
   extern __shared__ __align__(16) float sm[];
@@ -302,22 +305,14 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
     }
   };
 
-  // Keys in [seen_lo, seen_hi) are seen by every row of the warp: all of a decode step's, unless there is a window or several
-  // queries.  A batch outside has to ask for each row, and a hidden key's value takes no part, not even with weight zero: it
-  // may hold anything (0 * inf).  Two bodies, because the questions in the loop cost more than the second body does: 32
-  // sequences x 32 heads of 2048 tokens in fp16 197 us with them and 184 without; 8 query heads to each of 8 kv heads, 2048
-  // e5m2 tokens in 12 splits 36.6 and 33.0.
-  int seen_lo = 0, seen_hi = t1;
-#pragma unroll
-  for (int r = 0; r < RW; r++) {
-    if (causal && qpos[r] >= 0) {
-      const int limit = causal_base + qpos[r] + 1;
-      seen_hi = min(seen_hi, limit);
-      if (a.window > 0) seen_lo = max(seen_lo, limit - a.window);
-    }
-  }
-  auto batch = [&](int base, auto seen_by_all) {
-    constexpr bool kAll = decltype(seen_by_all)::value;
+  // (rows past the last one are worked out too: nothing reads them)
+  auto sees = [&](int pos, int r) {
+    if (!HIDES || !causal) return true;
+    const int limit = causal_base + qpos[r] + 1;
+    return pos < limit && (a.window <= 0 || pos >= limit - a.window);
+  };
+
+  for (int base = t0 + tsub * 4; base < t1; base += kPF * stride) {
     float sc[kPF][RW];
 #pragma unroll
     for (int i = 0; i < kPF; i++) {
@@ -346,7 +341,6 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
 #pragma unroll
         for (int r = 0; r < RW; r++) sc[i][r] += __shfl_xor_sync(0xffffffffu, sc[i][r], o);
     float corr[RW];
-    uint32_t hidden = 0;                                 // bit i * RW + r: the row does not see the step's key
 #pragma unroll
     for (int r = 0; r < RW; r++) {
       float mn = m[r];
@@ -355,15 +349,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
         const int pos = base + i * stride + tg;
         float s = sc[i][r];
         if (cap > 0.f) s = cap * tanhf(s * inv_cap_scaled);
-        bool ok = pos < t1;
-        if constexpr (!kAll) {
-          if (causal) {
-            const int limit = causal_base + qpos[r] + 1;
-            ok = ok && pos < limit && (a.window <= 0 || pos >= limit - a.window);
-          }
-          if (!ok) hidden |= 1u << (i * RW + r);
-        }
-        sc[i][r] = ok ? s : -INFINITY;
+        sc[i][r] = pos < t1 && sees(pos, r) ? s : -INFINITY;
         mn = fmaxf(mn, sc[i][r]);
       }
       const float ref = mn == -INFINITY ? 0.f : mn;      // nothing visible yet: every weight is zero
@@ -385,16 +371,14 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
       const int np = base + (kPF + i) * stride + tg;
       if (np < t1) vq[i].load(vc, head_off + (int64_t)np * a.c_s);
       else vq[i].clear();
+      // a hidden key's value takes no part, not even with weight zero: it may hold anything (0 * inf)
+      const int pos = base + i * stride + tg;
 #pragma unroll
       for (int r = 0; r < RW; r++)
 #pragma unroll
         for (int d = 0; d < DPL; d++)
-          if (kAll || ((hidden >> (i * RW + r)) & 1) == 0) acc[r][d] += sc[i][r] * vf[d];
+          if (sees(pos, r)) acc[r][d] += sc[i][r] * vf[d];
     }
-  };
-  for (int base = t0 + tsub * 4; base < t1; base += kPF * stride) {
-    if (base >= seen_lo && min(t1, base + kPF * stride) <= seen_hi) batch(base, std::true_type());
-    else batch(base, std::false_type());
   }
   // ---- new tokens (mode A, last split) from shared memory ----
   if (modeA && last_split) {
@@ -547,22 +531,17 @@ cudaError_t launch_rw(const AttnArgs& a, cudaStream_t s, bool pdl) {
     return (size_t)((modeA ? 2 * a.Sq * D : 0) + kAttnWarps * RW * D + kAttnWarps * RW * 2 +
                     2 * kMaxRows * a.nsplit + kMaxRows /* merge: weights, row sums */) * sizeof(float);
   };
-  if (rows <= 1) {
-    auto k = attn_decode_kernel<T, FP8, D, 1>;
-    size_t sm = smem_for(1);
+  const bool hides = a.window > 0 || (!modeA && a.causal && a.Sq > 1);
+  auto go = [&](auto rw) {
+    constexpr int RW = decltype(rw)::value;
+    auto k = hides ? attn_decode_kernel<T, FP8, D, RW, true> : attn_decode_kernel<T, FP8, D, RW, false>;
+    const size_t sm = smem_for(RW);
     if (sm > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     return launch_kernel(k, grid, dim3(kAttnThreads), sm, s, pdl, a);
-  } else if (rows <= 8 && !(rows > 4 && wide_rows())) {
-    auto k = attn_decode_kernel<T, FP8, D, 2>;
-    size_t sm = smem_for(2);
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    return launch_kernel(k, grid, dim3(kAttnThreads), sm, s, pdl, a);
-  } else {
-    auto k = attn_decode_kernel<T, FP8, D, 4>;
-    size_t sm = smem_for(4);
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    return launch_kernel(k, grid, dim3(kAttnThreads), sm, s, pdl, a);
-  }
+  };
+  if (rows <= 1) return go(std::integral_constant<int, 1>());
+  if (rows <= 8 && !(rows > 4 && wide_rows())) return go(std::integral_constant<int, 2>());
+  return go(std::integral_constant<int, 4>());
 }
 
 template <typename T, bool FP8>
@@ -598,9 +577,9 @@ IPEX_API int ipex_attn_decode_ctas_per_sm(int D, int rows, int fp8_kv, int dtype
     constexpr int kD = decltype(d)::value;
     const int r = min(kMaxRows, rows);
     const int rw = r <= 1 ? 1 : (r <= 8 && !(r > 4 && wide_rows())) ? 2 : 4;
-    const void* k = rw == 1   ? (const void*)attn_decode_kernel<T, kF, kD, 1>
-                    : rw == 2 ? (const void*)attn_decode_kernel<T, kF, kD, 2>
-                              : (const void*)attn_decode_kernel<T, kF, kD, 4>;
+    const void* k = rw == 1   ? (const void*)attn_decode_kernel<T, kF, kD, 1, false>
+                    : rw == 2 ? (const void*)attn_decode_kernel<T, kF, kD, 2, false>
+                              : (const void*)attn_decode_kernel<T, kF, kD, 4, false>;
     int n = 0;
     const size_t sm = (size_t)(2 * kD + kAttnWarps * rw * (kD + 2) + 33 * kMaxRows) * sizeof(float);
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kAttnThreads, sm) == cudaSuccess ? n : 0;
