@@ -90,7 +90,7 @@ __device__ __forceinline__ uint32_t at_rank(uint32_t smem_addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
   return a;
 }
-// Values to another CTA's shared memory, counted in bytes by a barrier there: no fence on either side.
+// Values to another CTA's shared memory, counted in bytes by a barrier there (the wait for it acquires at cluster scope).
 __device__ __forceinline__ void st_async2(uint32_t addr, uint32_t bar, float a, float b) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(a),
                "f"(b), "r"(bar)
@@ -337,8 +337,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tm_x, const FewArgs a) {
   uint64_t* d_full = empty + kStages;
   uint64_t* d_empty = d_full + C::kBufs;
   uint64_t* p_full = d_empty + C::kBufs;                                 // the parts of a tile have arrived
-  uint64_t* p_empty = p_full + 2;                                        // every CTA has read what this one sent it
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_empty + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint32_t* book = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(full) + 512);
 
@@ -359,10 +358,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tm_x, const FewArgs a) {
       mbar_init(&d_full[i], 1);
       mbar_init(&d_empty[i], 4);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&p_full[i], 1);
-      mbar_init(&p_empty[i], kSplit * 4);
-    }
+    for (int i = 0; i < 2; ++i) mbar_init(&p_full[i], 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -540,8 +536,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tm_x, const FewArgs a) {
       // ---- parts of the tile: rank q adds up and stores tokens [q * tq, (q + 1) * tq) ----
       const int pb = it & 1;
       const uint32_t pph = (it >> 1) & 1;
-      ok = warp_wait(&p_empty[pb], pph ^ 1, abort_flag);
-      if (!ok) break;
+      // The buffer is free: whoever sent the parts of tile it - 1, all of which this warp has waited for, had read those of tile
+      // it - 2 before.
       if (warp == 2 && elect_one()) mbar_expect_tx(&p_full[pb], (uint32_t)(kSplit * kBM * tq * 4));
       const uint32_t mine = smem_u32(part + (size_t)pb * C::kPart + ((size_t)rank * kBM + row) * tq);
 #pragma unroll
@@ -566,7 +562,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tm_x, const FewArgs a) {
         pdl_wait();                                 // out and residual belong to the kernels before this one until here
         waited = true;
       }
-      ok = warp_wait(&p_full[pb], pph, abort_flag);
+      ok = warp_wait<true>(&p_full[pb], pph, abort_flag);
       if (!ok) break;
       const int m0 = (int)rank * tq;
       const float* got = part + (size_t)pb * C::kPart + (size_t)row * tq;
@@ -589,8 +585,6 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tm_x, const FewArgs a) {
         }
       }
       __syncwarp();
-      if (lane < kSplit)
-        asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(at_rank(smem_u32(&p_empty[pb]), lane)) : "memory");
     }
     if (!ok && lane == 0) report(a.err, 22);
     __syncwarp();

@@ -42,27 +42,46 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
+// What is read or overwritten behind a wait was written or read in front of the arrivals, by this CTA or (CLUSTER) also by
+// another one of its cluster.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(b)), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(b)), "r"(parity)
+        : "memory");
   return ok != 0;
+}
+// Arrival at a barrier of another CTA of the cluster, by its cluster address.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 constexpr uint32_t kSpinLimit = 1u << 21;  // x (try_wait + up to 256 ns sleep): roughly half a second
 
 // Bounded wait.  Returns false when the limit ran out (and raises the CTA's abort flag) or when another role of the
 // CTA has already raised it.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t it = 0; it < kSpinLimit; ++it) {
-    if (mbar_try_wait(b, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(b, parity)) return true;
     if (it >= 64) {
       __nanosleep(it >= 4096 ? 256 : 32);
       if (*abort_flag) return false;
@@ -95,8 +114,9 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 // A bounded wait by a whole warp, the same answer in every lane.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(b, parity, abort_flag));
+  return __all_sync(0xffffffffu, mbar_wait<CLUSTER>(b, parity, abort_flag));
 }
 
 // ------------------------------------------------------------------------------------------------ TMA
