@@ -17,7 +17,8 @@
 //   warps 6..17  (packed weights) three teams of four expand units of 128 k in turn (a lane owns a weight row), so that a
 //                team has the time of six stages for the loads, arithmetic, stores and proxy fences of two; the next
 //                unit's bytes are already on their way to registers when a unit is begun, across tiles too.
-// All barriers that the MMA issuer waits for live in the leading CTA; the other CTA's warps arrive there remotely.
+// All barriers that the MMA issuer waits for live in the leading CTA; the other CTA's expanders count bytes there (send_token),
+// its epilogue arrives there remotely.  Waits for what another CTA of the cluster says acquire at cluster scope.
 // Every mbarrier wait is bounded; on expiry a role raises its CTA's abort flag, records a code in the error flag
 // (16 loader, 17 MMA issuer, 18 epilogue, 19 dequantizer) and leaves its loop; the CTAs meet before TMEM is released.
 #include <cuda.h>
@@ -83,8 +84,15 @@ __device__ __forceinline__ uint32_t leader_addr(const void* p) {   // the same s
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
   return a;
 }
-__device__ __forceinline__ void mbar_arrive_at(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// 16 bytes of this CTA's shared memory to the leading CTA, counted by a barrier there.  This is how the other CTA says that a
+// stage is filled: an arrival released at cluster scope waits some 1400 clocks for itself (by the thread that filled the stage
+// 1024 x 12288 x 4096 int4 77 -> 95 us, by a warp that does nothing else 172), while the copy runs behind the proxy fence by
+// itself, and completes with a release at that scope.
+constexpr uint32_t kTokenBytes = 16;
+__device__ __forceinline__ void send_token(uint32_t to, const void* from, uint32_t leader_bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to),
+               "r"(smem_u32(from)), "r"(kTokenBytes), "r"(leader_bar)
+               : "memory");
 }
 // Tile load into this CTA's shared memory whose bytes are counted by a barrier of the leading CTA.
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* tm, int x, int y, uint32_t leader_bar) {
@@ -147,7 +155,7 @@ __device__ __forceinline__ void ldg_nc_32b(const void* p, uint4& a, uint4& b) {
 // ---- dequantizers: fill the weight operand of every stage for this CTA's tiles ---------------------------------------
 template <typename T, int BT, int WF>
 __device__ __forceinline__ void expand_role(const PairArgs& a, uint8_t* sA, uint64_t* full, uint64_t* empty,
-                                            volatile int* abort_flag, const uint32_t* lut2) {
+                                            volatile int* abort_flag, const uint32_t* lut2, uint32_t token) {
   using C = PairCfg<BT>;
   using V = V2<T>;
   constexpr bool k4 = PairFam<WF>::four_bit;
@@ -235,7 +243,7 @@ __device__ __forceinline__ void expand_role(const PairArgs& a, uint8_t* sA, uint
       Scale<T> sc;
       sc.d = V::splat(scale(g == 0 ? cur.d0 : cur.d1));
       if constexpr (WF == WF_ASYM_INT4) sc.m = V::splat(scale(g == 0 ? cur.m0 : cur.m1));
-      if (ok && !warp_wait(&empty[s + g], ph ^ 1, abort_flag)) {
+      if (ok && !warp_wait<true>(&empty[s + g], ph ^ 1, abort_flag)) {
         if (lane == 0) report(a.err, 19);
         ok = false;
       }
@@ -262,7 +270,8 @@ __device__ __forceinline__ void expand_role(const PairArgs& a, uint8_t* sA, uint
       asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(kTeamThreads) : "memory");
       if (r == 0 && ok) {
         fence_proxy_async_smem();
-        mbar_arrive_at(full0 + (s + g) * 8);
+        if (rank == 0) mbar_arrive(&full[s + g]);
+        else send_token(token, sA + (s + g) * C::kABytes, full0 + (s + g) * 8);
       }
     }
     s += kStep;
@@ -293,7 +302,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   uint64_t* empty = full + C::kStages;
   uint64_t* acc_full = empty + C::kStages;
   uint64_t* acc_empty = acc_full + 2;                                                 // used in the leading CTA
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* token = acc_empty + 2;                                                    // written in the leading CTA, never read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(token + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint32_t* lut2 = reinterpret_cast<uint32_t*>(smem + C::kStages * C::kStageBytes + 256);
 
@@ -305,7 +315,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
-      mbar_init(&full[s], kDense ? 1 : 3);                             // the loader, and one team of each CTA
+      mbar_init(&full[s], kDense ? 1 : 2);                             // the loader, and the leading CTA's team
       mbar_init(&empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -342,13 +352,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     for (int t = first; t < ntiles && ok; t += tstep) {
       const int nb = t / a.m_tiles, mb = t % a.m_tiles;
       for (int kb = 0; kb < kblocks; ++kb) {
-        if (!warp_wait(&empty[s], ph ^ 1, abort_flag)) {
+        if (!warp_wait<true>(&empty[s], ph ^ 1, abort_flag)) {
           ok = false;
           break;
         }
         if (elect_one()) {
           // the leader expects the bytes of both CTAs; the other's may land first, the phase still waits for the arrivals
-          if (rank == 0) mbar_expect_tx(&full[s], 2 * (kDense ? C::kStageBytes : C::kBBytes));
+          if (rank == 0) mbar_expect_tx(&full[s], kDense ? 2 * C::kStageBytes : 2 * C::kBBytes + kTokenBytes);
           if constexpr (kDense)
             tma_load_2d_pair(sA + s * C::kABytes, &tm_w, kb * kBK, (nb * 2 + (int)rank) * kBM, full0 + s * 8);
           tma_load_2d_pair(sB + s * C::kBBytes, &tm_x, kb * kBK, row0 + mb * BT + (int)rank * (BT / 2), full0 + s * 8);
@@ -377,11 +387,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       for (int t = first; t < ntiles && ok; t += tstep, ++it) {
         const int acc = it & 1;
         const uint32_t acc_ph = (it >> 1) & 1;
-        ok = warp_wait(&acc_empty[acc], acc_ph ^ 1, abort_flag);
+        ok = warp_wait<true>(&acc_empty[acc], acc_ph ^ 1, abort_flag);
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BT;
         for (int kb = 0; kb < kblocks && ok; ++kb) {
-          if (!warp_wait(&full[s], ph, abort_flag)) {
+          if (!warp_wait<true>(&full[s], ph, abort_flag)) {
             ok = false;
             break;
           }
@@ -419,7 +429,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       // activation mode: lanes 0..15 hold gate rows, lanes 16..31 the matching up rows; 16 outputs per warp
       const int n_out = a.act != 0 ? nw / 2 + (lane & 15) : n;
       const bool writer = a.act != 0 ? (lane < 16 && n_out < a.N / 2) : (n < a.N);
-      if (!warp_wait(&acc_full[acc], acc_ph, abort_flag)) {
+      if (!warp_wait<true>(&acc_full[acc], acc_ph, abort_flag)) {
         if (lane == 0) report(a.err, 18);
         break;
       }
@@ -458,10 +468,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       }
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_at(acc_empty0 + acc * 8);
+      if (lane == 0) mbar_arrive_cluster(acc_empty0 + acc * 8);
     }
   } else {
-    if constexpr (!kDense) expand_role<T, BT, WF>(a, sA, full, empty, abort_flag, lut2);
+    if constexpr (!kDense) expand_role<T, BT, WF>(a, sA, full, empty, abort_flag, lut2, leader_addr(token));
   }
   tcgen05_fence_before();
   __syncthreads();
