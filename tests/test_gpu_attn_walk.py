@@ -65,6 +65,39 @@ def test_hidden_values_do_not_count(kind, heads, monkeypatch):
             assert torch.equal(out[:, :, rows], ref[:, :, rows]), (S, n)
 
 
+@pytest.mark.parametrize("heads", [(4, 4, 1), (8, 2, 3), (16, 1, 1)])               # one, twelve and sixteen rows a head
+@pytest.mark.parametrize("kind", ["half", "e5m2"])
+@pytest.mark.parametrize("window,cap", [(0, 5.0), (1, 0.0), (50, 0.0), (50, 5.0)])
+def test_walk_with_window_and_cap(window, cap, kind, heads, monkeypatch):
+    from ipex_llm_b200.ops import cuda_ops
+    Hq, Hkv, Sq = heads
+    D, dtype, u = 128, torch.float16, 2.0 ** -11
+    g = torch.Generator(device="cuda").manual_seed(Hq + window)
+    for S in (3, 16, 49, 65, 130, 520):
+        q = torch.randn(2, Hq, Sq, D, device="cuda", generator=g).to(dtype) * 3
+        k, v = (torch.randn(2, Hkv, S, D, device="cuda", generator=g).to(dtype) for _ in range(2))
+        kk, vv = k, v
+        if kind == "e5m2":
+            k, v = cuda_ops.quantize_kv_e5m2(k), cuda_ops.quantize_kv_e5m2(v)
+            kk, vv = cuda_ops.dequantize_kv_e5m2(k, dtype), cuda_ops.dequantize_kv_e5m2(v, dtype)
+        kd, vd = (t.double().repeat_interleave(Hq // Hkv, 1) for t in (kk, vv))
+        s = q.double() @ kd.transpose(-1, -2) / math.sqrt(D)
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        last = torch.arange(S - Sq, S, device="cuda")[:, None]
+        key = torch.arange(S, device="cuda")[None]
+        hidden = (key > last) | ((key <= last - window) if window else False)
+        p = torch.softmax(s.masked_fill(hidden, float("-inf")), -1)
+        ref = p @ vd
+        # as above; a capped score carries tanh's error too (2^-22 of the cap, in front of the exponential)
+        bound = ref.abs() * u + (p @ vd.abs()) * 2.0 ** -17 + 1e-7
+        for n in (1, 2, 8):
+            monkeypatch.setattr(cuda_ops, "attn_splits", lambda *a, n=n: n)
+            out = cuda_ops.sdpa_decode(q, k, v, None, 1.0 / math.sqrt(D), cap, window)
+            torch.cuda.synchronize()
+            assert bool(((out.double() - ref).abs() <= bound).all()), (S, n)
+
+
 def test_splits_fit_the_gpu(monkeypatch):
     from ipex_llm_b200.ops import cuda_ops
     monkeypatch.delenv("IPEX_LLM_ATTN_STEPS", raising=False)

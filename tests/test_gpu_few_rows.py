@@ -175,3 +175,57 @@ def test_batch_whose_weights_begin_at_16_bytes():
 
     want, got = step(False), step(True)
     assert float((got - want).norm() / want.norm()) < 8 * 2.0 ** -11
+
+
+# the first four go to the product for few rows, the last two are formats that it would round and stay with the others
+@pytest.mark.parametrize("name,dtype", [("sym_int4", torch.float16), ("nf4", torch.float16), ("fp8_e4m3", torch.bfloat16),
+                                        ("sym_int8", torch.bfloat16), ("asym_int4", torch.float16), ("nf4", torch.bfloat16)])
+@pytest.mark.parametrize("M,K", [(5, 8320), (7, 11008), (8, 8320)])
+def test_long_rows_between_dependent_launches(name, dtype, M, K):
+    """Five to eight rows of a long contraction: against float64, and in a chain of programmatic launches whose buffers are
+    overwritten by the next round."""
+    from ipex_llm_b200.ops import cuda_ops, tcgen05_gemm
+    from ipex_llm_b200.quant import qtypes
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    N = 272
+    few = tcgen05_gemm.few_exact(cuda_ops.QTYPE_TO_WF[qtypes.qtype_from_name(name)], dtype, M)
+    assert few == (name != "asym_int4" and (name, dtype) != ("nf4", torch.bfloat16))
+    qu, pu, _ = _weights("sym_int4", K, 384, dtype, g)            # makes the long rows, the same ones every time
+    q, packed, w = _weights(name, N, K, dtype, g)
+    bias = torch.randn(N, device="cuda", generator=g).to(dtype)
+    start = torch.randn(M, 384, device="cuda", generator=g).to(dtype)
+    x, y, y2, z = (torch.empty(M, n, dtype=dtype, device="cuda") for n in (K, N, N, 384))
+
+    def chain(pdl):
+        z.copy_(start)
+        seen = []
+        for _ in range(4):
+            # the long rows made, read, made again in the same place and read again, beside the first result
+            for rows, out, res in ((z, y, z[:, :N]), (start, y2, y)):
+                cuda_ops.gemv_lowbit(rows, pu, qu, K, 384, out=x, pdl=pdl)
+                cuda_ops.gemv_lowbit(x, packed, q, N, K, out=out, bias=bias, residual=res, pdl=pdl)
+                if not pdl:
+                    seen.append((x.clone(), res.clone(), out.clone()))
+            z[:, :N].copy_(y2 * 0.1)
+        return y2.clone(), seen
+
+    want, seen = chain(False)
+    torch.cuda.synchronize()
+    got, _ = chain(True)
+    torch.cuda.synchronize()
+    cuda_ops.check_error_flag(x.device)
+    if few:
+        assert torch.equal(got, want)                             # (kernels that add parts up in any order do not repeat)
+    # what a product rounds: see the bounds of the product for few rows above; kernels for one to eight rows hold x in 15 bits
+    for xs, zs, ys in seen:
+        ref = xs.double() @ w.t() + bias.double() + zs.double()
+        mag = xs.double().abs() @ w.abs().t()
+        top = xs.double().abs().amax(1, keepdim=True) * w.abs().sum(1)
+        bound = mag * ((8 if name == "asym_int4" else 1) * U[dtype] + K * 2.0 ** -23) + top * 2.0 ** -14 + \
+            (ref.abs() + 1e-3) * U[dtype]
+        assert bool(((ys.double() - ref).abs() <= bound).all())
+    moved = cuda_ops.gemv_lowbit(x, _at_16_bytes(packed), q, N, K, bias=bias, residual=z[:, :N])
+    torch.cuda.synchronize()
+    ref = x.double() @ w.t() + bias.double() + z[:, :N].double()
+    top = x.double().abs().amax(1, keepdim=True) * w.abs().sum(1)
+    assert bool(((moved.double() - ref).abs() <= top * 2.0 ** -10 + ref.abs() * U[dtype]).all())
