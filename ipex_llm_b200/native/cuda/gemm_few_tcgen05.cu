@@ -80,16 +80,6 @@ template <int BT, int WF, bool CODES> struct FewCfg {
 };
 
 // ---- cluster helpers ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t few_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t at_rank(uint32_t smem_addr, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
-  return a;
-}
 // Values to another CTA's shared memory, counted in bytes by a barrier there (the wait for it acquires at cluster scope).
 __device__ __forceinline__ void st_async2(uint32_t addr, uint32_t bar, float a, float b) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(a),
@@ -100,9 +90,6 @@ __device__ __forceinline__ void st_async4(uint32_t addr, uint32_t bar, float a, 
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
                "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar)
                : "memory");
-}
-__device__ __forceinline__ void cluster_meet() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // 32 lanes x N columns, without the wait
 template <int N> __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, float* v) {
@@ -179,16 +166,6 @@ __device__ __forceinline__ float group_scale(uint32_t raw) {
   else return __uint_as_float(raw) * (Fp8Place<T, WF>::mul * Fp8Place<T, WF>::pre);
 }
 
-__device__ __forceinline__ uint32_t few_ldg_u16(const void* p) {
-  uint16_t v;
-  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ void few_ldg_32b(const void* p, uint4& a, uint4& b) {
-  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-               : "l"(p));
-}
 
 // ---- expanders ------------------------------------------------------------------------------------------------------
 template <typename T, int BT, int WF, bool CODES>
@@ -233,18 +210,18 @@ __device__ __forceinline__ void few_expand(const FewArgs& a, int u_begin, int u_
     n.q[0] = n.q[1] = n.q[2] = n.q[3] = make_uint4(0, 0, 0, 0);
     n.d0 = n.d1 = n.m0 = n.m1 = 0;
     if (valid) {
-      few_ldg_32b(wp, n.q[0], n.q[1]);
-      few_ldg_32b(wp + 32, n.q[2], n.q[3]);
+      ldg_nc_32b(wp, n.q[0], n.q[1]);
+      ldg_nc_32b(wp + 32, n.q[2], n.q[3]);
       if constexpr (!CODES && k4) {
-        n.d0 = few_ldg_u16(sp);
-        n.d1 = few_ldg_u16(sp + 16);
+        n.d0 = ldg_nc_u16(sp);
+        n.d1 = ldg_nc_u16(sp + 16);
         if constexpr (WF == WF_ASYM_INT4) {
           const uint16_t* mp = sp + a.Np * (a.Kp / 64);
-          n.m0 = few_ldg_u16(mp);
-          n.m1 = few_ldg_u16(mp + 16);
+          n.m0 = ldg_nc_u16(mp);
+          n.m1 = ldg_nc_u16(mp + 16);
         }
       } else if constexpr (!CODES) {
-        n.d0 = few_ldg_u16(sp + lp * 16);           // int8: a piece is a scale's 64 k
+        n.d0 = ldg_nc_u16(sp + lp * 16);           // int8: a piece is a scale's 64 k
       }
     }
     if (++lp == kPieces) {
@@ -342,7 +319,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tm_x, const FewArgs a) {
   uint32_t* book = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(full) + 512);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const uint32_t rank = few_rank();
+  const uint32_t rank = cta_rank();
   const int first = blockIdx.x / kSplit, tstep = gridDim.x / kSplit;
   // this CTA's share of every tile's k, in stages of 128
   const int k128 = (int)(a.Kp / 128);
@@ -372,7 +349,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tm_x, const FewArgs a) {
   if (warp == 1) tmem_alloc(tmem_slot, C::kTmemCols);
   tcgen05_fence_before();
   __syncthreads();
-  cluster_meet();
+  cluster_sync_all();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -485,7 +462,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tm_x, const FewArgs a) {
         for (int g = 0; g < kGroups; ++g) {
           x.d[g] = 0;
           if (kCodes && valid && i < nfold) {
-            if constexpr (FewFam<WF, CODES>::half_scale) x.d[g] = few_ldg_u16(sc16 + srow + (i * 2 + g) * 16);
+            if constexpr (FewFam<WF, CODES>::half_scale) x.d[g] = ldg_nc_u16(sc16 + srow + (i * 2 + g) * 16);
             else x.d[g] = ldg_nc_u32(sc32 + srow + i * 16);
           }
         }
@@ -594,7 +571,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tm_x, const FewArgs a) {
   pdl_launch_dependents();
   tcgen05_fence_before();
   __syncthreads();
-  cluster_meet();                                   // no CTA leaves while another may still write into it
+  cluster_sync_all();                                   // no CTA leaves while another may still write into it
   if (warp == 1) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, C::kTmemCols);

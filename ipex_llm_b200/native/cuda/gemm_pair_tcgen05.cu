@@ -71,19 +71,6 @@ template <int BT> struct PairCfg {
 };
 
 // ---- two-CTA forms ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cta_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t leader_addr(const void* p) {   // the same shared-memory variable in the leading CTA
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
-  return a;
-}
 // 16 bytes of this CTA's shared memory to the leading CTA, counted by a barrier there.  This is how the other CTA says that a
 // stage is filled: an arrival released at cluster scope waits some 1400 clocks for itself (by the thread that filled the stage
 // 1024 x 12288 x 4096 int4 77 -> 95 us, by a warp that does nothing else 172), while the copy runs behind the proxy fence by
@@ -140,17 +127,6 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&v)[16])
       : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ uint32_t ldg_nc_u16(const void* p) {
-  uint16_t v;
-  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
-  return v;
-}
-// 32 bytes of one weight row in one request (two 16-byte loads would fetch each sector twice)
-__device__ __forceinline__ void ldg_nc_32b(const void* p, uint4& a, uint4& b) {
-  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-               : "l"(p));
-}
 
 // ---- dequantizers: fill the weight operand of every stage for this CTA's tiles ---------------------------------------
 template <typename T, int BT, int WF>
@@ -175,7 +151,7 @@ __device__ __forceinline__ void expand_role(const PairArgs& a, uint8_t* sA, uint
   const float* sc32 = reinterpret_cast<const float*>(planes);
   const uint16_t* mins = sc16 + a.Np * (a.Kp / 64);
   const int prow = pair_row(r & 15);
-  const uint32_t full0 = leader_addr(full);
+  const uint32_t full0 = at_rank(smem_u32(full), 0);
 
   // where the next load stands: tile, unit, and the row it belongs to
   int lt = blockIdx.x >> 1, lu = team;
@@ -345,7 +321,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       if constexpr (kDense) prefetch_tmap(&tm_w);
       prefetch_tmap(&tm_x);
     }
-    const uint32_t full0 = leader_addr(full);
+    const uint32_t full0 = at_rank(smem_u32(full), 0);
     int s = 0;
     uint32_t ph = 0;
     bool ok = true;
@@ -417,7 +393,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     T* out = reinterpret_cast<T*>(a.out);
     const T* res = reinterpret_cast<const T*>(a.residual);
     const T* bias = reinterpret_cast<const T*>(a.bias);
-    const uint32_t acc_empty0 = leader_addr(acc_empty);
+    const uint32_t acc_empty0 = at_rank(smem_u32(acc_empty), 0);
     int it = 0;
     for (int t = first; t < ntiles; t += tstep, ++it) {
       const int nb = t / a.m_tiles, mb = t % a.m_tiles;
@@ -471,7 +447,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       if (lane == 0) mbar_arrive_cluster(acc_empty0 + acc * 8);
     }
   } else {
-    if constexpr (!kDense) expand_role<T, BT, WF>(a, sA, full, empty, abort_flag, lut2, leader_addr(token));
+    if constexpr (!kDense) expand_role<T, BT, WF>(a, sA, full, empty, abort_flag, lut2, at_rank(smem_u32(token), 0));
   }
   tcgen05_fence_before();
   __syncthreads();

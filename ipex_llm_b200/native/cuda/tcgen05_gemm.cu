@@ -562,11 +562,15 @@ cudaError_t launch_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const Gemm
 template <typename T, int WF>
 cudaError_t dispatch_bt(int bt, const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs& a, int sms,
                         cudaStream_t st) {
-  switch (bt) {
-    case 32: return launch_gemm<T, 32, WF>(tw, tx, a, sms, st);
-    case 64: return launch_gemm<T, 64, WF>(tw, tx, a, sms, st);
-    case 128: return launch_gemm<T, 128, WF>(tw, tx, a, sms, st);
-    default: return launch_gemm<T, 256, WF>(tw, tx, a, sms, st);
+  if (bt == 32) return launch_gemm<T, 32, WF>(tw, tx, a, sms, st);
+  if constexpr (Fam<WF>::dense) {      // more than 64 rows of dense weights always run on pairs
+    return launch_gemm<T, 64, WF>(tw, tx, a, sms, st);
+  } else {
+    switch (bt) {
+      case 64: return launch_gemm<T, 64, WF>(tw, tx, a, sms, st);
+      case 128: return launch_gemm<T, 128, WF>(tw, tx, a, sms, st);
+      default: return launch_gemm<T, 256, WF>(tw, tx, a, sms, st);
+    }
   }
 }
 
@@ -616,8 +620,7 @@ IPEX_API int ipex_gemm_few_tcgen05(const void* x, const void* w, void* out, cons
 // packed weights (the dequantizers' share does not shrink), 0.6 with dense ones.
 static int pair_tile(int M, int N, bool dense, const void* w) {
   if (M <= 64 || (!dense && (reinterpret_cast<uintptr_t>(w) & 31))) return 0;
-  const int pairs = sm_count() / 2;
-  if (pairs < 1) return 0;
+  const int pairs = sm_count() / 2 > 1 ? sm_count() / 2 : 1;
   const int64_t nt = (N + 255) / 256;
   const int64_t w256 = ((M + 255) / 256 * nt + pairs - 1) / pairs, w128 = ((M + 127) / 128 * nt + pairs - 1) / pairs;
   return (dense ? 0.6 : 0.77) * (double)w128 < (double)w256 ? 128 : 256;
@@ -715,7 +718,9 @@ IPEX_API int ipex_gemm_lowbit_tcgen05_grouped(const void* x, const void* w, void
   if (wf == WF_LUT4 && lut == nullptr) return (int)cudaErrorInvalidValue;
   if (bt != 32 && bt != 64 && bt != 128 && bt != 256) return (int)cudaErrorInvalidValue;
   if (wf < WF_SYM_INT4 || wf > WF_INT8) return (int)cudaErrorInvalidValue;
-  if (bt >= 128 && (reinterpret_cast<uintptr_t>(w) & 31) == 0)   // as for one matrix: the pair wins at every such size
+  // As for one matrix, also where many experts have few tokens or none: the whole bank, int4, 8 experts of 4096 x 14336 with
+  // 260 / 1024 tokens 2269 -> 1267 / 3088 -> 2014 us, 64 experts of 2048 x 1408 with 2048 tokens (four each) 4847 -> 3349.
+  if (bt >= 128 && (reinterpret_cast<uintptr_t>(w) & 31) == 0)
     return ipex_gemm_pair_tcgen05_grouped(x, w, out, lut, m_range, M_total, m_upper, N, K, ldx, ldo, wf, act, dtype, bt, err,
                                           stream);
   const CUtensorMapDataType tdt = dtype == DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;

@@ -468,6 +468,11 @@ def pick_nsplit(B: int, Hkv: int, kv_len: int, n_sm: int = 148, rows: int = 1) -
 
 
 @functools.lru_cache(maxsize=None)
+def _sm_count() -> int:
+    return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+
+
+@functools.lru_cache(maxsize=None)
 def _attn_ctas_per_sm(head_dim: int, rows: int, fp8: bool, dtype_code: int) -> int:
     return max(1, int(cuda_lib().ipex_attn_decode_ctas_per_sm(head_dim, min(rows, 16), int(fp8), dtype_code)))
 
@@ -484,8 +489,9 @@ def attn_splits(B: int, Hkv: int, kv_len: int, rows: int, head_dim: int, fp8: bo
     if "IPEX_LLM_ATTN_STEPS" in os.environ or "IPEX_LLM_ATTN_MIN_CTAS" in os.environ:
         return pick_nsplit(B, Hkv, kv_len, rows=rows)
     heads = B * Hkv * -(-max(1, rows) // 16)
-    wave = 148 * _attn_ctas_per_sm(head_dim, max(1, rows), bool(fp8), api.dtype_code(dtype)) // heads
-    if heads >= 148:
+    sms = _sm_count()
+    wave = sms * _attn_ctas_per_sm(head_dim, max(1, rows), bool(fp8), api.dtype_code(dtype)) // heads
+    if heads >= sms:
         n = kv_len // 512
     else:
         n = max(4, kv_len // 160) if kv_len >= (192 if rows <= 1 else 96) else 1

@@ -102,9 +102,9 @@ FEW_MAX_ROWS = 64      # rows of x (two per token when it comes in pairs) that g
 
 
 def few_exact(wf: int, dtype, rows: int) -> bool:
-    """Whether ``gemm_few`` multiplies by the codes of this format without rounding them (``rows`` of x up to 32, or pairs):
-    then it is at least as precise as the kernels for one to eight rows.  A code book's values round to bf16, a format with
-    minima is expanded to 16 bits."""
+    """Whether ``gemm_few`` is at least as precise as the kernels for one to eight rows (``rows`` of x up to 32, or pairs): it
+    multiplies by the codes, which it does not round, or by a code book's values in fp16, as they do.  In bf16 a code book's
+    values would round to fewer bits than there, and a format with minima is expanded to 16 bits."""
     if wf == api.WF_ASYM_INT4 or (wf == api.WF_LUT4 and dtype != torch.float16):
         return False
     return rows <= 32

@@ -9,6 +9,7 @@ def _engine(monkeypatch, n_heads, n_kv, prompt, batch=1, max_len=4096):
     monkeypatch.delenv("IPEX_LLM_ATTN_STEPS", raising=False)
     monkeypatch.delenv("IPEX_LLM_ATTN_MIN_CTAS", raising=False)
     monkeypatch.setattr(cuda_ops, "_attn_ctas_per_sm", lambda *a: 2)
+    monkeypatch.setattr(cuda_ops, "_sm_count", lambda: 148)
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     eng = DecoderEngine.__new__(DecoderEngine)
     eng.n_heads, eng.n_kv, eng.hd, eng.kv_fp8, eng.dtype, eng.max_len = n_heads, n_kv, 128, True, torch.float16, max_len
@@ -67,6 +68,7 @@ def test_few_splits_are_four(monkeypatch):
     monkeypatch.delenv("IPEX_LLM_ATTN_STEPS", raising=False)
     monkeypatch.delenv("IPEX_LLM_ATTN_MIN_CTAS", raising=False)
     monkeypatch.setattr(cuda_ops, "_attn_ctas_per_sm", lambda *a: 2)
+    monkeypatch.setattr(cuda_ops, "_sm_count", lambda: 148)
     for Hkv, rows, start in ((32, 1, 192), (8, 8, 96), (2, 7, 96), (1, 1, 192)):
         got = [cuda_ops.attn_splits(1, Hkv, kv, rows, 128, True, torch.float16) for kv in range(1, 5000)]
         assert got[:start - 1] == [1] * (start - 1) and got[start - 1] == 4 and got == sorted(got)
