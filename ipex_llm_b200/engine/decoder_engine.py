@@ -463,7 +463,8 @@ class DecoderEngine:
         if 8 < B <= 24 and self._few_decode_ok():
             # some sequences: the weights are read once per step (eight-row GEMVs read them once per group of eight).  The
             # normalised rows come as value and remainder and the products multiply by the codes themselves (a code book's
-            # values in fp16, as the GEMVs), so nothing is rounded that the GEMVs would not round.  Llama-2-7B sym_int4, 16 sequences: 7.16 -> 4.91 ms per step.
+            # values in fp16, as the GEMVs), so nothing is rounded that the GEMVs would not round.  Llama-2-7B sym_int4, 16
+            # sequences: 7.16 -> 4.91 ms per step.
             for L in self.layers:
                 self._few(L.qkv, cuda_ops.rms_norm_pairs(h0, L.ln1, self.eps), self.qkv_buf[:B], pairs=True)
                 self._attention(L, B)

@@ -615,7 +615,7 @@ IPEX_API int ipex_gemm_few_tcgen05(const void* x, const void* w, void* out, cons
 
 // Token tile of the pair kernel for this product, 0 where the kernel of this file keeps it.  Up to 64 tokens its narrower
 // tiles (32, 64) do less work on padding.  Above, the pair wins at every size measured (int4, K = 4096: 128 x 4096 61.5 ->
-// 37 us, 128 x 12288 62 -> 41, 1024 x 4096 59 -> 31, 1024 x 12288 138 -> 78, 4096 x 22016 788 -> 495; dense fp16 1024 x
+// 37 us, 128 x 12288 62 -> 41, 1024 x 4096 59 -> 31, 1024 x 12288 138 -> 79, 4096 x 22016 788 -> 495; dense fp16 1024 x
 // 12288 96 -> 81).  Between its tiles the count of waves decides: a k block of 128 tokens costs 0.77 of one of 256 with
 // packed weights (the dequantizers' share does not shrink), 0.6 with dense ones.
 static int pair_tile(int M, int N, bool dense, const void* w) {
@@ -681,7 +681,7 @@ IPEX_API int ipex_gemm_lowbit_tcgen05(const void* x, const void* w, void* out, c
   if (wf < WF_SYM_INT4 || wf > WF_INT8) return (int)cudaErrorInvalidValue;
   if (const int pt = pair_tile(M, N, false, w))
     return ipex_gemm_pair_tcgen05(x, w, out, bias, residual, lut, M, N, K, ldx, 0, ldo, ldr, wf, act, dtype, pt, err, stream);
-  // up to 64 rows: int4 at 32 rows 12288 x 4096 41.7 -> 23.3 us, 4096 x 4096 38.6 -> 11.5, 22016 x 4096 84 -> 40, 4096 x 11008
+  // up to 64 rows: int4 at 32 rows 12288 x 4096 41.7 -> 22.7 us, 4096 x 4096 38.6 -> 11.8, 22016 x 4096 84 -> 39, 4096 x 11008
   // 97 -> 19
   if (M <= 64 && (reinterpret_cast<uintptr_t>(w) & 31) == 0)
     return ipex_gemm_few_tcgen05(x, w, out, bias, residual, lut, M, N, K, ldx, ldo, ldr, wf, act, 0, dtype, 0, err, stream);
