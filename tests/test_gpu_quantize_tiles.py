@@ -56,3 +56,22 @@ def test_slices_between_other_bytes():
     assert bool((buf[:4] == 0xA5).all()) and bool((buf[-4:] == 0xA5).all())
     dense = dequantize_device(packed, (40, 256), qt.SYM_INT4, torch.float16)
     assert torch.equal(dequantize_device(part, (40, 256), qt.SYM_INT4, torch.float16), dense)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("name", ["sym_int4", "fp8_e4m3"])
+def test_expand_into_rows_of_any_alignment(name, dtype):
+    """Rows at multiples of 32, 16 and fewer bytes take stores of their own width, and leave the gaps between them alone."""
+    from ipex_llm_b200.native import cuda_api as api
+    from ipex_llm_b200.native.lib import cuda_lib, current_stream, ptr
+    from ipex_llm_b200.ops.cuda_ops import QTYPE_TO_WF, dequantize_device
+    from ipex_llm_b200.ops.cuda_quant import quantize_to_device_layout
+    from ipex_llm_b200.quant import qtypes as qt
+    N, K, q = 37, 384, qt.qtype_from_name(name)
+    packed = quantize_to_device_layout(torch.randn(N, K, device="cuda").half(), q)
+    dense = dequantize_device(packed, (N, K), q, dtype)
+    for gap in (0, 32, 16 // dense.element_size(), 3):
+        buf = torch.full((N, K + gap), 7.0, dtype=dtype, device="cuda")
+        rc = cuda_lib().ipex_dequantize_tiles(ptr(packed), ptr(buf), N, K, K + gap, QTYPE_TO_WF[q], None, api.dtype_code(dtype),
+                                              current_stream())
+        assert rc == 0 and torch.equal(buf[:, :K], dense) and bool((buf[:, K:] == 7.0).all())
