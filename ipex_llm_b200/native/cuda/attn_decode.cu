@@ -157,9 +157,12 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
   using Raw = RawKV<T, FP8, DPL>;
   constexpr int kStepWords = 2 * Raw::kWords;            // registers one step in flight holds
   constexpr int kState = 2 * RW * DPL;                   // registers of the q rows and their accumulators
-  constexpr int kBudget = kState <= 64 ? 64 : (kState <= 128 ? 32 : 16);
+  // With several rows a warp the words in flight are held to what leaves an SM its warps: 8 sequences x 32 heads of 128, four
+  // queries, 4000 fp16 tokens 496 us four deep, 311 two deep.  Rows of 256 by fours spill whatever the depth: a kv head of 32
+  // such rows, 1500 fp16 tokens 307 us two deep, 247 with a step at a time.
+  constexpr int kBudget = RW == 1 ? 64 : kState <= 128 ? 32 : 16;
   constexpr int kWant = kBudget / kStepWords;
-  constexpr int kPF = kWant >= 4 ? 4 : 2;
+  constexpr int kPF = kWant >= 4 ? 4 : kWant >= 2 ? 2 : 1;
   int chunk = (past + a.nsplit - 1) / a.nsplit;
   chunk = (chunk + 15) & ~15;
   const int t0 = split * chunk;
