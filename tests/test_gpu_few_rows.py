@@ -190,6 +190,7 @@ def test_long_rows_between_dependent_launches(name, dtype, M, K):
     N = 272
     few = tcgen05_gemm.few_exact(cuda_ops.QTYPE_TO_WF[qtypes.qtype_from_name(name)], dtype, M)
     assert few == (name != "asym_int4" and (name, dtype) != ("nf4", torch.bfloat16))
+    few = few and (name in ("sym_int4", "fp8_e4m3") or M * K >= 1 << 16)      # fewer of the others fit beside their kernel's rings
     qu, pu, _ = _weights("sym_int4", K, 384, dtype, g)            # makes the long rows, the same ones every time
     q, packed, w = _weights(name, N, K, dtype, g)
     bias = torch.randn(N, device="cuda", generator=g).to(dtype)
