@@ -487,7 +487,8 @@ def attn_splits(B: int, Hkv: int, kv_len: int, rows: int, head_dim: int, fp8: bo
     1024 11.3 us at 8 splits, 12.3 at 11, 13.1 at 3).  Handing over costs the same for two parts as for four, so a walk that
     is split at all is split in four: 32 heads of 128 tokens 7.6 us whole, 9.5 in two, 9.3 in four, of 256 tokens 10.2, 10.7
     and 9.6; 8 kv heads of 8 rows, whose warps divide the rows and walk all tokens, 64 tokens 16.2, 18.9 and 17.1, 128 tokens
-    21.0, 21.3 and 18.4.  ``pick_nsplit``'s rule, which knows the walk's length only, where its switches ask for it."""
+    21.0, 21.3 and 18.4.  Rows of 256 by fours pay
+    from 96 tokens on: their steps are slow (a kv head of 32 such rows, 1500 fp16 tokens 247 us in eight parts, 201 in twelve).  ``pick_nsplit``'s rule, which knows the walk's length only, where its switches ask for it."""
     if "IPEX_LLM_ATTN_STEPS" in os.environ or "IPEX_LLM_ATTN_MIN_CTAS" in os.environ:
         return pick_nsplit(B, Hkv, kv_len, rows=rows)
     heads = B * Hkv * -(-max(1, rows) // 16)
@@ -496,7 +497,7 @@ def attn_splits(B: int, Hkv: int, kv_len: int, rows: int, head_dim: int, fp8: bo
     if heads >= sms:
         n = kv_len // 512
     else:
-        n = max(4, kv_len // 160) if kv_len >= (192 if rows <= 1 else 96) else 1
+        n = max(4, kv_len // (160 if head_dim <= 128 or rows <= 8 else 96)) if kv_len >= (192 if rows <= 1 else 96) else 1
     # a captured step keeps its count: few different ones, so that prompts of similar length share a graph
     return max(c for c in (1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128) if c <= max(1, min(n, wave)))
 

@@ -74,3 +74,6 @@ def test_few_splits_are_four(monkeypatch):
         assert got[:start - 1] == [1] * (start - 1) and got[start - 1] == 4 and got == sorted(got)
     assert cuda_ops.attn_splits(3, 32, 400, 1, 128, True, torch.float16) == 3        # what fits at once
     assert cuda_ops.attn_splits(8, 32, 400, 1, 128, True, torch.float16) == 1
+    # rows of 256 by fours take shorter walks
+    assert [cuda_ops.attn_splits(1, 1, 700, rows, D, True, torch.float16) for rows, D in ((8, 256), (16, 128), (16, 256))] == \
+        [4, 4, 6]
