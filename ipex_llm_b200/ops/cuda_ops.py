@@ -108,8 +108,8 @@ def gemv_lowbit(x: torch.Tensor, w_data: torch.Tensor, qtype: int, N: int, K: in
         out = torch.empty((M, n_out), dtype=x.dtype, device=x.device)
     lut = lut_for(qtype, x.device) if wf == api.WF_LUT4 else None
     if M > 4 and K > 8192 and (M * K >= 1 << 16 or wf in (api.WF_SYM_INT4, api.WF_FP8_E4M3)) and K % 128 == 0 and \
-            N % 16 == 0 and norm_weight is None and act == 0 and wf not in (api.WF_F16, api.WF_BF16) and x.dtype in (torch.float16, torch.bfloat16) and \
-            out.dtype == x.dtype and out.stride(1) == 1 and _GEMV_IMPL == "stream":
+            N % 16 == 0 and norm_weight is None and act == 0 and wf not in (api.WF_F16, api.WF_BF16) and \
+            x.dtype in (torch.float16, torch.bfloat16) and out.dtype == x.dtype and out.stride(1) == 1 and _GEMV_IMPL == "stream":
         # five to eight long rows do not fit beside the rings of the kernels below, which then stream the weights twice or
         # leave the rings: 4096 x 11008 at 8 rows, int4 33.8 -> 18.8 us, fp8 36.6 -> 25.1, nf4 143 -> 27.6.  (Up to 128 KB of
         # rows do fit beside the rings of the formats that the streaming kernel does not take: 2048 x 11008 at 5 rows, nf4
@@ -487,8 +487,9 @@ def attn_splits(B: int, Hkv: int, kv_len: int, rows: int, head_dim: int, fp8: bo
     1024 11.3 us at 8 splits, 12.3 at 11, 13.1 at 3).  Handing over costs the same for two parts as for four, so a walk that
     is split at all is split in four: 32 heads of 128 tokens 7.6 us whole, 9.5 in two, 9.3 in four, of 256 tokens 10.2, 10.7
     and 9.6; 8 kv heads of 8 rows, whose warps divide the rows and walk all tokens, 64 tokens 16.2, 18.9 and 17.1, 128 tokens
-    21.0, 21.3 and 18.4.  Rows of 256 by fours pay
-    from 96 tokens on: their steps are slow (a kv head of 32 such rows, 1500 fp16 tokens 247 us in eight parts, 201 in twelve).  ``pick_nsplit``'s rule, which knows the walk's length only, where its switches ask for it."""
+    21.0, 21.3 and 18.4.  Rows of 256 by fours pay from 96 tokens on: their steps are slow (a kv head of 32 such rows, 1500
+    fp16 tokens 247 us in eight parts, 201 in twelve).  ``pick_nsplit``'s rule, which knows the walk's length only, where its
+    switches ask for it."""
     if "IPEX_LLM_ATTN_STEPS" in os.environ or "IPEX_LLM_ATTN_MIN_CTAS" in os.environ:
         return pick_nsplit(B, Hkv, kv_len, rows=rows)
     heads = B * Hkv * -(-max(1, rows) // 16)
