@@ -460,20 +460,23 @@ class DecoderEngine:
                                     current_stream())
             api.check(rc, "embedding")
         # (later pipeline stages: the previous stage's hidden states were received into h[0][:B])
-        if 8 < B <= 24 and self._few_decode_ok():
-            # some sequences: the weights are read once per step (eight-row GEMVs read them once per group of eight).  The
-            # normalised rows come as value and remainder and the products multiply by the codes themselves (a code book's
-            # values in fp16, as the GEMVs), so nothing is rounded that the GEMVs would not round.  Llama-2-7B sym_int4, 16
-            # sequences: 7.16 -> 4.91 ms per step.
+        if B <= 24 and self._few_decode_ok() and B >= self._few_from:
+            # some sequences (formats without a streaming GEMV: any number): the weights are read once per step (eight-row GEMVs read them once per group of eight, and work
+            # the rows up in every CTA).  The normalised rows come as value and remainder and the products multiply by the codes
+            # themselves (a code book's values in fp16, as the GEMVs), so nothing is rounded that the GEMVs would not round.
+            # Llama-2-7B sym_int4, 8 sequences of 517 tokens: 3.15 -> 2.74 ms per step; four of its layers, one sequence of 512
+            # tokens, nf4: 477 -> 403 us, sym_int8: 422 -> 364; four sequences, nf4: 541 -> 422, but sym_int4: 351 -> 362.
+            def pairs(h, w):
+                return cuda_ops.rms_norm_pairs(h, w, self.eps, pdl=self.use_pdl)
             for L in self.layers:
-                self._few(L.qkv, cuda_ops.rms_norm_pairs(h0, L.ln1, self.eps), self.qkv_buf[:B], pairs=True)
+                self._few(L.qkv, pairs(h0, L.ln1), self.qkv_buf[:B], pairs=True)
                 self._attention(L, B)
                 self._few(L.o, self.attn_buf[:B], h1, residual=h0)
-                self._few(L.gate_up, cuda_ops.rms_norm_pairs(h1, L.ln2, self.eps), self.act_buf[:B], act=1, pairs=True)
+                self._few(L.gate_up, pairs(h1, L.ln2), self.act_buf[:B], act=1, pairs=True)
                 self._few(L.down, self.act_buf[:B], h0, residual=h1)
             if self.last_stage:
                 if self.lm_gather is None:
-                    self._few(self.lm_head, cuda_ops.rms_norm_pairs(h0, self.final_norm, self.eps), self.logits[:B], pairs=True)
+                    self._few(self.lm_head, pairs(h0, self.final_norm), self.logits[:B], pairs=True)
                 else:
                     self._lm_head(h0, B)
                 rc = lib.ipex_argmax(ptr(self.logits), ptr(self.tokens), B, self.vocab, self.logits.stride(0), dtc, pdl,
@@ -485,20 +488,20 @@ class DecoderEngine:
             # many sequences: every projection is one tcgen05 low-bit product that reads the weights once per step.
             # Llama-2-7B sym_int4, 32 sequences of 256 tokens: 13.0 -> 5.0 ms per step.
             for L in self.layers:
-                x = cuda_ops.rms_norm(h0, L.ln1, self.eps)
-                self._gemm(L.qkv, x, out=self.qkv_buf[:B])
+                x = cuda_ops.rms_norm(h0, L.ln1, self.eps, pdl=self.use_pdl)
+                self._gemm_step(L.qkv, x, out=self.qkv_buf[:B])
                 self._attention(L, B)
-                self._gemm(L.o, self.attn_buf[:B], residual=h0, out=h1)
+                self._gemm_step(L.o, self.attn_buf[:B], residual=h0, out=h1)
                 if L.moe is not None:
                     self._moe_mlp(L, h1, h0)
                     continue
-                x = cuda_ops.rms_norm(h1, L.ln2, self.eps)
-                self._gemm(L.gate_up, x, act=1, out=self.act_buf[:B])
-                self._gemm(L.down, self.act_buf[:B], residual=h1, out=h0)
+                x = cuda_ops.rms_norm(h1, L.ln2, self.eps, pdl=self.use_pdl)
+                self._gemm_step(L.gate_up, x, act=1, out=self.act_buf[:B])
+                self._gemm_step(L.down, self.act_buf[:B], residual=h1, out=h0)
             if self.last_stage:
-                x = cuda_ops.rms_norm(h0, self.final_norm, self.eps)
+                x = cuda_ops.rms_norm(h0, self.final_norm, self.eps, pdl=self.use_pdl)
                 if self.lm_gather is None:
-                    self._gemm(self.lm_head, x, out=self.logits[:B])
+                    self._gemm_step(self.lm_head, x, out=self.logits[:B])
                 else:
                     off, n = self.vocab_offset, self.lm_head.N
                     self.logits[:B, off:off + n].copy_(self._gemm(self.lm_head, x))
@@ -604,8 +607,8 @@ class DecoderEngine:
             os.environ.get("IPEX_LLM_DECODE_GEMM", "1") != "0"
 
     def _few_decode_ok(self) -> bool:
-        """Decode steps of nine to 24 sequences on the product for few rows: formats it multiplies by without rounding them,
-        weights that begin at 32 bytes (the GEMVs take 16), no experts, one GPU."""
+        """Decode steps of up to 24 sequences on the product for few rows: formats it multiplies by without rounding them,
+        weights that begin at 32 bytes (the GEMVs take 16), no experts, one GPU.  ``_few_from``: from as many sequences on."""
         from ..ops import tcgen05_gemm
         ok = self.__dict__.get("_few_ok")
         if ok is None:
@@ -614,14 +617,26 @@ class DecoderEngine:
                 all(w is not None and w.K % 128 == 0 and w.N % 16 == 0 and w.wf not in (api.WF_F16, api.WF_BF16) and
                     w.data.data_ptr() % 32 == 0 and tcgen05_gemm.few_exact(w.wf, self.dtype, 1) for w in ws)
             self._few_ok = ok
+            self._few_from = 5 if any(w is not None and w.wf in (api.WF_SYM_INT4, api.WF_FP8_E4M3) for w in ws) else 1
         return ok
 
     def _few(self, w: _W, x, out, residual=None, act=0, pairs=False):
         from ..ops import tcgen05_gemm
         lut = cuda_ops.lut_for(w.qtype, x.device) if w.wf == api.WF_LUT4 else None
         if not tcgen05_gemm.gemm_few(x, w.data, w.N, w.K, out, w.wf, lut=lut, bias=w.bias, residual=residual, act=act,
-                                     pairs=pairs):
+                                     pairs=pairs, pdl=self.use_pdl):
             raise RuntimeError("decode engine: operands of the few-row product are not aligned")
+
+    def _gemm_step(self, w: _W, x, out, residual=None, act=0):
+        """``_gemm`` for the rows of a decode step: up to 64 go to the product for few rows, launched while its predecessor ends."""
+        from ..ops import tcgen05_gemm
+        if w.tp is None and w.wf not in (api.WF_F16, api.WF_BF16) and w.K % 128 == 0 and (act == 0 or w.N % 32 == 0) and \
+                x.shape[0] <= tcgen05_gemm.FEW_MAX_ROWS:
+            lut = cuda_ops.lut_for(w.qtype, x.device) if w.wf == api.WF_LUT4 else None
+            if tcgen05_gemm.gemm_few(x, w.data, w.N, w.K, out, w.wf, lut=lut, bias=w.bias, residual=residual, act=act,
+                                     pdl=self.use_pdl):
+                return
+        self._gemm(w, x, residual=residual, act=act, out=out)
 
     def _flat_prefill_ok(self) -> bool:
         ok = self.__dict__.get("_flat_ok")

@@ -608,10 +608,10 @@ IPEX_API int ipex_gemm_pair_tcgen05(const void* x, const void* w, void* out, con
 IPEX_API int ipex_gemm_pair_tcgen05_grouped(const void* x, const void* w, void* out, const float* lut, const int* m_range,
                                             int M_total, int m_upper, int N, int K, int64_t ldx, int64_t ldo, int wf, int act,
                                             int dtype, int bt, int* err, void* stream);
-// gemm_few_tcgen05.cu: packed weights with up to 64 rows.
-IPEX_API int ipex_gemm_few_tcgen05(const void* x, const void* w, void* out, const void* bias, const void* residual,
-                                   const float* lut, int M, int N, int K, int64_t ldx, int64_t ldo, int64_t ldr, int wf,
-                                   int act, int pairs, int dtype, int pdl, int* err, void* stream);
+// gemm_few.cu: packed weights with up to 64 rows.
+IPEX_API int ipex_gemm_few(const void* x, const void* w, void* out, const void* bias, const void* residual, const float* lut,
+                           int M, int N, int K, int64_t ldx, int64_t ldo, int64_t ldr, int wf, int act, int pairs, int dtype,
+                           int pdl, int split, int* err, void* stream);
 
 // Token tile of the pair kernel for this product, 0 where the kernel of this file keeps it.  Up to 64 tokens its narrower
 // tiles (32, 64) do less work on padding.  Above, the pair wins at every size measured (int4, K = 4096: 128 x 4096 61.5 ->
@@ -681,10 +681,10 @@ IPEX_API int ipex_gemm_lowbit_tcgen05(const void* x, const void* w, void* out, c
   if (wf < WF_SYM_INT4 || wf > WF_INT8) return (int)cudaErrorInvalidValue;
   if (const int pt = pair_tile(M, N, false, w))
     return ipex_gemm_pair_tcgen05(x, w, out, bias, residual, lut, M, N, K, ldx, 0, ldo, ldr, wf, act, dtype, pt, err, stream);
-  // up to 64 rows: int4 at 32 rows 12288 x 4096 41.7 -> 22.7 us, 4096 x 4096 38.6 -> 11.8, 22016 x 4096 84 -> 39, 4096 x 11008
-  // 97 -> 19
-  if (M <= 64 && (reinterpret_cast<uintptr_t>(w) & 31) == 0)
-    return ipex_gemm_few_tcgen05(x, w, out, bias, residual, lut, M, N, K, ldx, ldo, ldr, wf, act, 0, dtype, 0, err, stream);
+  // up to 64 rows: int4 at 32 rows 12288 x 4096 41.7 -> 21.5 us, 4096 x 4096 38.6 -> 10.6, 22016 x 4096 84 -> 33.7, 4096 x
+  // 11008 97 -> 17.7
+  if (M <= 64 && K % 128 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0)
+    return ipex_gemm_few(x, w, out, bias, residual, lut, M, N, K, ldx, ldo, ldr, wf, act, 0, dtype, 0, 0, err, stream);
   const int bt = ipex_gemm_tcgen05_token_tile(M);
   const CUtensorMapDataType tdt = dtype == DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUtensorMap tx;

@@ -107,16 +107,12 @@ def gemv_lowbit(x: torch.Tensor, w_data: torch.Tensor, qtype: int, N: int, K: in
     if out is None:
         out = torch.empty((M, n_out), dtype=x.dtype, device=x.device)
     lut = lut_for(qtype, x.device) if wf == api.WF_LUT4 else None
-    if M > 4 and K > 8192 and (M * K >= 1 << 16 or wf in (api.WF_SYM_INT4, api.WF_FP8_E4M3)) and K % 128 == 0 and \
-            N % 16 == 0 and norm_weight is None and act == 0 and wf not in (api.WF_F16, api.WF_BF16) and \
-            x.dtype in (torch.float16, torch.bfloat16) and out.dtype == x.dtype and out.stride(1) == 1 and _GEMV_IMPL == "stream":
-        # five to eight long rows do not fit beside the rings of the kernels below, which then stream the weights twice or
-        # leave the rings: 4096 x 11008 at 8 rows, int4 33.8 -> 18.8 us, fp8 36.6 -> 25.1, nf4 143 -> 27.6.  (Up to 128 KB of
-        # rows do fit beside the rings of the formats that the streaming kernel does not take: 2048 x 11008 at 5 rows, nf4
-        # 24.6 us there and 32.8 here, int8 22.6 and 26.6; at 6 rows 113 and 32.8, 112 and 26.7.)
+    if norm_weight is None and wf not in (api.WF_F16, api.WF_BF16) and _GEMV_IMPL == "stream" and act in (0, 1, 2) and \
+            (act == 0 or (N % 32 == 0 and residual is None)) and K % (128 if wf in (api.WF_FP8_E4M3, api.WF_FP8_E5M2) else 64) == 0:
         from . import tcgen05_gemm
-        if tcgen05_gemm.few_exact(wf, x.dtype, M) and \
-                tcgen05_gemm.gemm_few(x, w_data, N, K, out, wf, lut=lut, bias=bias, residual=residual, pdl=pdl and _USE_PDL):
+        if tcgen05_gemm.few_faster(wf, x.dtype, M) and \
+                tcgen05_gemm.gemm_few(x, w_data, N, K, out, wf, lut=lut, bias=bias, residual=residual, act=act,
+                                      pdl=pdl and _USE_PDL):
             return out
     if _GEMV_IMPL == "stream" and wf in (api.WF_SYM_INT4, api.WF_FP8_E4M3) and x.stride(0) % 8 == 0 and \
             getattr(lib, "ipex_gemv_lowbit_stream", None) is not None:

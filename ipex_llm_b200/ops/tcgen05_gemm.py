@@ -104,16 +104,28 @@ FEW_MAX_ROWS = 64      # rows of x (two per token when it comes in pairs) that g
 def few_exact(wf: int, dtype, rows: int) -> bool:
     """Whether ``gemm_few`` is at least as precise as the kernels for one to eight rows (``rows`` of x up to 32, or pairs): it
     multiplies by the codes, which it does not round, or by a code book's values in fp16, as they do.  In bf16 a code book's
-    values would round to fewer bits than there, and a format with minima is expanded to 16 bits."""
+    values would round to fewer bits than there; a format with minima is expanded to 16 bits beyond 32 rows."""
     if wf == api.WF_ASYM_INT4 or (wf == api.WF_LUT4 and dtype != torch.float16):
         return False
     return rows <= 32
 
 
+def few_faster(wf: int, dtype, rows: int) -> bool:
+    """Whether ``gemm_few`` takes one to eight rows instead of the GEMVs: it loses no precision (see ``few_exact``; minima are
+    kept apart up to 32 rows) and is faster.  The streaming GEMV of int4 and e4m3 keeps up to three rows.  us, GEMV / this, 4096
+    x 4096 | 12288 x 4096 | 4096 x 11008: int4 one row 5.5 / 5.3 | 10.2 / 11.6 | 10.1 / 10.4, four 7.3 / 5.7 | 11.7 / 11.9 | 15.4
+    / 10.6, eight 11.1 / 6.4 | 16.9 / 12.3 | -; one row in nf4 8.8 / 6.4 | 20.1 / 14.4 | 16.9 / 12.3, int8 7.4 / 6.2 | 16.1 /
+    11.9 | 14.3 / 11.2.  (Two or three rows of int4 win by themselves where N is small, and lose it again where the two kinds
+    take turns: a decode step of four layers, two sequences, 321 us with GEMVs alone and 327 with both.)"""
+    if wf == api.WF_LUT4 and dtype != torch.float16:
+        return False
+    return rows >= 4 or wf not in (api.WF_SYM_INT4, api.WF_FP8_E4M3)
+
+
 def gemm_few(x: torch.Tensor, w_data: torch.Tensor, N: int, K: int, out: torch.Tensor, wf: int, lut: torch.Tensor = None,
              bias: torch.Tensor = None, residual: torch.Tensor = None, act: int = 0, pairs: bool = False,
-             pdl: bool = False) -> bool:
-    """``x @ dequant(w).T`` for few rows into ``out`` (see native/cuda/gemm_few_tcgen05.cu); ``pairs``: ``x`` holds value and
+             pdl: bool = False, split: int = 0) -> bool:
+    """``x @ dequant(w).T`` for few rows into ``out`` (see native/cuda/gemm_few.cuh); ``pairs``: ``x`` holds value and
     remainder of every token in turn (``cuda_ops.rms_norm_pairs``).  False, and nothing is launched, when the operands do not
     suit the kernel."""
     M, n_out = out.shape[0], N // 2 if act else N
@@ -129,12 +141,12 @@ def gemm_few(x: torch.Tensor, w_data: torch.Tensor, N: int, K: int, out: torch.T
                                  residual.shape[1] < n_out or residual.stride(1) != 1):
         return False
     lib = cuda_lib()
-    rc = lib.ipex_gemm_few_tcgen05(ptr(x), ptr(w_data), ptr(out), ptr(bias), ptr(residual), ptr(lut), M, N, K, x.stride(0),
-                                   out.stride(0), residual.stride(0) if residual is not None else 0, wf, int(act), int(pairs),
-                                   api.dtype_code(x.dtype), int(pdl), ptr(_err(x.device)), current_stream())
+    rc = lib.ipex_gemm_few(ptr(x), ptr(w_data), ptr(out), ptr(bias), ptr(residual), ptr(lut), M, N, K, x.stride(0),
+                           out.stride(0), residual.stride(0) if residual is not None else 0, wf, int(act), int(pairs),
+                           api.dtype_code(x.dtype), int(pdl), split, ptr(_err(x.device)), current_stream())
     if rc == -1:
         raise RuntimeError("ipex_llm_b200: the driver's tensor-map encoder rejected the GEMM operands")
-    api.check(rc, "gemm_few_tcgen05")
+    api.check(rc, "gemm_few")
     return True
 
 

@@ -65,6 +65,45 @@ def test_few_rows(name, shape, dtype):
         assert torch.equal(out, again)
 
 
+@pytest.mark.parametrize("split", range(9))
+@pytest.mark.parametrize("shape", [(1, 16, 64), (3, 144, 192), (8, 272, 832), (31, 160, 1088), (40, 400, 2112)])
+@pytest.mark.parametrize("name", ["sym_int4", "asym_int4", "nf4", "sym_int8"])
+def test_few_rows_shared_by_any_number(name, shape, split):
+    """Every number of CTAs to a tile's k (0: chosen), k that ends in half a chunk of 128; minima up to 32 rows are not rounded."""
+    from ipex_llm_b200.ops import cuda_ops, tcgen05_gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(K)
+    q, packed, w = _weights(name, N, K, torch.float16, g)
+    x = torch.randn(M, K, device="cuda", generator=g).half()
+    out = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+    assert tcgen05_gemm.gemm_few(x, packed, N, K, out, cuda_ops.QTYPE_TO_WF[q], lut=cuda_ops.lut_for(q, x.device), split=split)
+    torch.cuda.synchronize()
+    cuda_ops.check_error_flag(x.device)
+    mag, ref = x.double().abs() @ w.abs().t(), x.double() @ w.t()
+    roundings = 1 if name == "nf4" else 8 if name == "asym_int4" and M > 32 else 0
+    # (the sums of a minimum's group cancel against those of its codes: up to the block's range times the tokens)
+    spread = x.double().abs().sum(1, keepdim=True) * 0.5 * K ** 0.5 * 2.0 ** -23 if name == "asym_int4" else 0.0
+    bound = mag * (roundings * U[torch.float16] + K * 2.0 ** -23) + spread + ref.abs() * U[torch.float16] + 1e-6
+    assert bool(((out.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("name,dtype", [("sym_int4", torch.float16), ("fp8_e4m3", torch.bfloat16), ("nf4", torch.float16),
+                                        ("nf4", torch.bfloat16), ("asym_int4", torch.float16), ("sym_int8", torch.bfloat16)])
+def test_one_to_eight_rows_by_either_way(name, dtype):
+    """``gemv_lowbit`` on both sides of its rule, and with operands that only the GEMVs take."""
+    from ipex_llm_b200.ops import cuda_ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for N in (528, 8208):
+        q, packed, w = _weights(name, N, 384, dtype, g)
+        for M in (1, 2, 4, 5, 8):
+            x = torch.randn(M, 384, device="cuda", generator=g).to(dtype)
+            ref = x.double() @ w.t()
+            top = x.double().abs().amax(1, keepdim=True) * w.abs().sum(1)
+            bound = top * 2.0 ** -10 + ref.abs() * U[dtype] + 1e-6 if dtype == torch.float16 else top * U[dtype] + ref.abs() * U[dtype]
+            for y in (cuda_ops.gemv_lowbit(x, packed, q, N, 384), cuda_ops.gemv_lowbit(x, _at_16_bytes(packed), q, N, 384)):
+                assert bool(((y.double() - ref).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("pairs", [False, True])
 @pytest.mark.parametrize("shape", [(9, 288, 256), (24, 4128, 512)])
 def test_few_rows_gated(shape, pairs):
