@@ -5,6 +5,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #define IPEX_API extern "C" __attribute__((visibility("default")))
 
 // activation dtype codes used across the C ABI
@@ -99,6 +101,22 @@ __device__ __forceinline__ uint32_t ldg_nc_u32(const void* p) {
   asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
+
+// A kernel's limit of dynamic shared memory, set once per device and kernel (one of these, static, beside each kernel's launch:
+// the call takes longer than the rest of a launch's preparation).
+struct SmemLimit {
+  std::atomic<uint64_t> done{0};
+  cudaError_t operator()(const void* kernel, int bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (dev < 64 && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+  }
+};
 
 // Host-side launch helper: plain launch or programmatic-dependent launch on `stream`.
 template <typename... KArgs, typename... Args>

@@ -453,7 +453,8 @@ template <typename T, int WF, int NT, int WN>
 int launch(const Operands& o, Args a, cudaStream_t st, bool pdl, int asked) {
   using C = Cfg<WF, NT, WN>;
   auto kern = kernel<T, WF, NT, WN>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+  static SmemLimit limit;
+  cudaError_t e = limit((const void*)kern, C::kSmem);
   if (e != cudaSuccess) return (int)e;
   const int tiles = (o.N + kBM - 1) / kBM;
   a.split = pick_split(tiles, (a.chunks + C::WK - 1) / C::WK, asked);

@@ -736,10 +736,9 @@ cudaError_t launch_stream(StreamArgs a, cudaStream_t stream, bool pdl) {
   a.cpw = p.cpw;
   a.wpt = p.wpt;
   auto kern = a.moe_ranges != nullptr ? gemv_stream_kernel<T, WFK, RT, 1, true> : gemv_stream_kernel<T, WFK, RT, MH, false>;
-  if (p.smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
-    if (e != cudaSuccess) return e;
-  }
+  static SmemLimit limit[2];
+  cudaError_t e = limit[a.moe_ranges != nullptr]((const void*)kern, 227 * 1024);
+  if (e != cudaSuccess) return e;
   return launch_kernel(kern, dim3(p.grid), dim3(kThreads), p.smem, stream, pdl, a);
 }
 

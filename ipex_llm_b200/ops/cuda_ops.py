@@ -176,11 +176,37 @@ def _gemv_rows_per_call(K: int, dtype_size: int = 2) -> int:
     return max(1, min(GEMV_MAX_M, (_SMEM_LIMIT - 8192) // ((kp + 8) * 2)))
 
 
+def _linear_rows(x: torch.Tensor, weight: FP4Params, M: int, N: int, K: int, wf: int):
+    """``lowbit_linear`` for up to 64 packed rows in one native call, or None where they need the general way."""
+    from . import tcgen05_gemm
+    if not x.is_contiguous() or x.shape[1] != K:
+        return None
+    few = M > GEMV_MAX_M or tcgen05_gemm.few_faster(wf, x.dtype, M)
+    if M > GEMV_MAX_M and (N % 16 != 0 or os.environ.get("IPEX_LLM_TCGEN05", "1") == "0"):
+        return None
+    lut = lut_for(weight.qtype, x.device) if wf == api.WF_LUT4 else None
+    out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    rc = cuda_lib().ipex_linear_rows(x.data_ptr(), weight.data_ptr(), out.data_ptr(), None if lut is None else lut.data_ptr(), M, N,
+                                     K, wf, api.DT_F16 if x.dtype == torch.float16 else api.DT_BF16, few,
+                                     error_flag(x.device).data_ptr(), current_stream())
+    if rc == 0:
+        return out
+    if rc != 1:
+        api.check(rc, "linear_rows")
+    return None
+
+
 def lowbit_linear(x: torch.Tensor, weight: FP4Params) -> torch.Tensor:
     """``x [M, K] @ dequant(weight).T`` for any qtype, any M."""
-    N, K = int(weight._shape[0]), int(weight._shape[1])
+    N, K = weight._shape
     qtype = weight.qtype
     M = x.shape[0]
+    wf = QTYPE_TO_WF.get(qtype)
+    if wf is not None and M <= 64 and (x.dtype is torch.float16 or x.dtype is torch.bfloat16) and _GEMV_IMPL == "stream":
+        out = _linear_rows(x, weight, M, N, K, wf)
+        if out is not None:
+            return out
+    N, K = int(N), int(K)
     if x.dtype == torch.float32:
         return lowbit_linear(x.to(torch.float16), weight).to(torch.float32)
     if is_tiled(qtype):

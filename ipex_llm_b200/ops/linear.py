@@ -103,6 +103,8 @@ class MatMulLowBitCPU(torch.autograd.Function):
 class LowBitLinear(nn.Linear):
     """``nn.Linear`` whose weight is an ``FP4Params`` of any block qtype."""
 
+    tp_gather = None      # found here, the look-up of a module that has no such group does not go through ``__getattr__``
+
     def __init__(self, input_features, output_features, qtype, bias=True, conver_to_half=True, mp_group=None,
                  optimize_lm_head=False, act_order=False, enable_scale_search=False):
         super().__init__(input_features, output_features, bias, device="meta")
@@ -156,20 +158,27 @@ class LowBitLinear(nn.Linear):
         # empty tensor support (MoE experts that receive no token)
         if self.training and x.requires_grad and self.compute_dtype is not None:
             x = x.to(self.compute_dtype)
-        if self.bias is not None and self.bias.dtype != x.dtype:
-            self.bias.data = self.bias.data.to(x.dtype)
+        params = self._parameters
+        bias = params["bias"] if "bias" in params else self.bias
+        if bias is not None and bias.dtype != x.dtype:
+            bias.data = bias.data.to(x.dtype)
         if self.optimize_lm_head and os.environ.get("IPEX_LLM_LAST_LM_HEAD", "1") != "0":
             x = reshape_lm_head_input(x)
         x_shape = x.shape
-        new_shape = x_shape[:-1] + (self.out_len,)
-        x_2d = x.contiguous().view(-1, x_shape[-1])
+        flat = len(x_shape) == 2
+        new_shape = None if flat else x_shape[:-1] + (self.out_len,)
+        x_2d = x.contiguous()
+        if not flat:
+            x_2d = x_2d.view(-1, x_shape[-1])
+        elif x_2d.requires_grad and not torch.is_grad_enabled():
+            x_2d = x_2d.detach()
         if self.act_order:
             x_2d = x_2d[:, self.g_idx_map]
-        w = self.weight
+        w = params["weight"] if "weight" in params else self.weight
         if x_2d.shape[0] == 0:
-            return torch.empty(new_shape, dtype=x.dtype, device=x.device)
+            return torch.empty(x_shape[:-1] + (self.out_len,), dtype=x.dtype, device=x.device)
         if x_2d.is_cuda:
-            if not (w.quantized and w.data.is_cuda):
+            if not (w.quantized and w.is_cuda):
                 raise RuntimeError("LowBitLinear: input is on cuda but the packed weight is not; call model.to('cuda')")
             if x_2d.requires_grad:
                 result = MatMulLowBit.apply(x_2d, w, self.out_len)
@@ -183,10 +192,11 @@ class LowBitLinear(nn.Linear):
                 result = cuda_ops.lowbit_linear(x_2d, w)
                 if low_mem:
                     torch.cuda.empty_cache()
-            result = result.view(new_shape)
+            if not flat:
+                result = result.view(new_shape)
             result = _all_reduce(result, self.mp_group)
-            if self.bias is not None:
-                result = result + self.bias
+            if bias is not None:
+                result = result + bias
             return _gather_last_dim(result, self)
         # CPU
         if not w.quantized:
@@ -199,7 +209,8 @@ class LowBitLinear(nn.Linear):
         else:
             result = ggml_matmul_src1_x_src0_t(w.data.view(torch.uint8) if w.data.dtype != torch.uint8 else w.data,
                                                x_2d, self.weight_shape, w.qtype).to(x.dtype)
-        result = result.view(new_shape)
+        if not flat:
+            result = result.view(new_shape)
         result = _all_reduce(result, self.mp_group)
         if self.bias is not None:
             result = result + self.bias

@@ -104,6 +104,29 @@ def test_one_to_eight_rows_by_either_way(name, dtype):
                 assert bool(((y.double() - ref).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("name", ["sym_int4", "nf4", "fp8_e4m3", "asym_int4"])
+def test_linear_of_any_rows(name):
+    """A packed linear layer on both sides of its one-call way: rows, a half chunk of k, odd outputs, shapes, rows apart."""
+    from ipex_llm_b200.ops.linear import LowBitLinear
+    from ipex_llm_b200.quant import qtypes as qt
+    from ipex_llm_b200.quant.params import FP4Params
+    g = torch.Generator(device="cuda").manual_seed(6)
+    K = 384 if name == "fp8_e4m3" else 192
+    for N in (16, 328):
+        layer = LowBitLinear(K, N, qt.qtype_from_name(name), bias=False)
+        w = (torch.randn(N, K, device="cuda", generator=g) * 0.05).half()
+        layer._parameters["weight"] = FP4Params(w, requires_grad=False, quantized=False, qtype=layer.qtype).to("cuda")
+        dense = layer.weight.dequantize(torch.float32).double()
+        for shape in ((1,), (3,), (8,), (9,), (64,), (65,), (2, 4), (0,), (1, 1, 5)):
+            x = torch.randn(*shape, K + 8, device="cuda", generator=g).half()[..., :K].requires_grad_()
+            with torch.no_grad():
+                y = layer(x)
+            assert y.shape == (*shape, N) and not y.requires_grad
+            ref = x.detach().double() @ dense.t()
+            top = x.detach().double().abs().sum(-1, keepdim=True) * float(dense.abs().max())
+            assert bool(((y.double() - ref).abs() <= top * 2.0 ** -10 + 1e-3).all())
+
+
 @pytest.mark.parametrize("pairs", [False, True])
 @pytest.mark.parametrize("shape", [(9, 288, 256), (24, 4128, 512)])
 def test_few_rows_gated(shape, pairs):
