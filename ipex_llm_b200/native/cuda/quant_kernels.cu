@@ -35,15 +35,46 @@ template <int N> __device__ __forceinline__ int nearest_sorted(const float* tabl
   return (v - table[lo] <= table[lo + 1] - v) ? lo : lo + 1;
 }
 
+// The same of sixteen values within [-1, 1] that lie more than 1 / 16 apart: a bucket of 1 / 32 holds one of them at most, so the
+// bucket names the value below it and the next one to ask for (two look-ups instead of five in a chain; 7008 x 6400 bf16 to
+// nf4 82 -> 56 us).
+struct Buckets {
+  float2 step[65];      // of a bucket: the next value, and the index of the one below it (as bits)
+  float2 pair[16];      // values i and i + 1
+  __device__ void fill(const float* values) {
+    for (int i = threadIdx.x; i < 65; i += blockDim.x) {
+      const float edge = (float)(i - 1) / 32.0f - 1.0f;         // a bucket's width below it: the product that picks it is rounded
+      int lo = 0;
+      for (int j = 1; j < 15; ++j)
+        if (values[j] <= edge) lo = j;
+      step[i] = make_float2(values[lo + 1], __int_as_float(lo));
+    }
+    for (int i = threadIdx.x; i < 15; i += blockDim.x) pair[i] = make_float2(values[i], values[i + 1]);
+  }
+  __device__ __forceinline__ int nearest(float v) const {
+    const float2 st = step[min(64, max(0, (int)__fmaf_rn(v, 32.0f, 32.0f)))];
+    const int lo = min(__float_as_int(st.y) + (st.x <= v ? 1 : 0), 14);
+    const float2 p = pair[lo];
+    return (v - p.x <= p.y - v) ? lo : lo + 1;
+  }
+};
+
 // Kinds of the tiled formats.
 enum { Q_SYM4 = 0, Q_ASYM4 = 1, Q_NF4 = 2, Q_FP4 = 3, Q_E4M3 = 4, Q_E5M2 = 5, Q_INT8 = 6 };
 
-// 64 consecutive elements of a row as raw words: 16-byte loads where the row allows it.
+// 64 consecutive elements of a row as raw words; `wide`: the bytes that every run's address is a multiple of (32, 16 or less).
 template <typename T> struct Run64 {
   static constexpr int kWords = 64 * (int)sizeof(T) / 4;
   uint32_t w[kWords];
-  __device__ __forceinline__ void load(const T* p, bool vec) {
-    if (vec) {
+  __device__ __forceinline__ void load(const T* p, int wide) {
+    if (wide == 32) {
+#pragma unroll
+      for (int i = 0; i < kWords; i += 8)
+        asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(w[i]), "=r"(w[i + 1]), "=r"(w[i + 2]), "=r"(w[i + 3]), "=r"(w[i + 4]), "=r"(w[i + 5]),
+                       "=r"(w[i + 6]), "=r"(w[i + 7])
+                     : "l"(reinterpret_cast<const uint32_t*>(p) + i));
+    } else if (wide == 16) {
 #pragma unroll
       for (int i = 0; i < kWords / 4; ++i) {
         const uint4 q = __ldg(reinterpret_cast<const uint4*>(p) + i);
@@ -67,22 +98,88 @@ template <typename T> struct Run64 {
       return DT<T>::to_f(*reinterpret_cast<const T*>(&h));
     }
   }
+  // Smallest and largest element; NaNs are left out, as fminf and fmaxf do (two 16-bit elements at a time).
+  __device__ __forceinline__ void extremes(float& lo, float& hi) const {
+    if constexpr (sizeof(T) == 4) {
+      lo = hi = at(0);
+#pragma unroll
+      for (int i = 1; i < 64; ++i) {
+        lo = fminf(lo, at(i));
+        hi = fmaxf(hi, at(i));
+      }
+    } else {
+      using T2 = std::conditional_t<std::is_same<T, __half>::value, __half2, __nv_bfloat162>;
+      T2 l = *reinterpret_cast<const T2*>(&w[0]), h = l;
+#pragma unroll
+      for (int i = 1; i < kWords; ++i) {
+        const T2 v = *reinterpret_cast<const T2*>(&w[i]);
+        l = __hmin2(l, v);
+        h = __hmax2(h, v);
+      }
+      lo = fminf(DT<T>::to_f(l.x), DT<T>::to_f(l.y));
+      hi = fmaxf(DT<T>::to_f(h.x), DT<T>::to_f(h.y));
+    }
+  }
+  // The first element of the largest magnitude, as a serial loop from element 0 on finds it.
+  __device__ __forceinline__ float first_largest(float lo, float hi) const {
+    const float first = at(0);
+    if (first != first) return first;                    // nothing compares above it
+    if (hi > -lo) return hi;
+    if (hi < -lo) return lo;
+    if (hi == 0.f) return first;                         // zeros of either sign
+    float top = first;                                   // both signs
+#pragma unroll
+    for (int i = 1; i < 64; ++i)
+      if (fabsf(at(i)) > fabsf(top)) top = at(i);
+    return top;
+  }
 };
+
+// (int)y within [0, 15] for a whole run of eight, nibble by nibble: the number in the last bits of 2^23 + y, rounded down (what
+// is not a number becomes zero, as the conversion has it).  put(k): the element whose code is nibble k.
+template <typename F> __device__ __forceinline__ uint32_t nibbles(F&& put) {
+  uint32_t w = 0;
+#pragma unroll
+  for (int k = 7; k >= 0; --k) {
+    const float y = fminf(fmaxf(put(k), 0.f), 15.5f);
+    w = w * 16 + (__float_as_uint(__fadd_rz(y, 8388608.f)) - 0x4B000000u);
+  }
+  return w;
+}
+
+// 32 bytes at an address that is a multiple of 16, or (`whole`) of 32.
+__device__ __forceinline__ void store32(uint8_t* to, uint4 a, uint4 b, bool whole) {
+  if (whole) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(to), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x),
+                 "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+  } else {
+    reinterpret_cast<uint4*>(to)[0] = a;
+    reinterpret_cast<uint4*>(to)[1] = b;
+  }
+}
 
 // Dense rows -> device tiles.  A warp makes one tile of 16 rows x 128 k, a lane one run of 64 in it (row lane / 2, half
 // lane & 1): the block's scale is found in the lane's own registers (fp8 blocks of 128: two lanes), without shuffles over
 // the warp, and a tile's codes leave as whole sectors.  Every byte is read and written once, padding included
-// (rows up to 16, k up to 128 are written as zeros).  Bounded by the requests: a lane's 16-byte accesses go along its own
-// run of 128 bytes, so a warp's access touches 32 runs.  11008 x 4096 fp16 to sym_int4, 17 us of bytes: 190 us (behind a 123
-// us copy to fp32 and a zero fill) with a warp per block and two elements a lane, 39 us now.
+// (rows up to 16, k up to 128 are written as zeros).  Bounded by its instructions, some eight for an element, and by the
+// requests: a lane's accesses go along its own run of 128 bytes, so a warp's access touches 32 runs, with 32 bytes to each.
+// 11008 x 4096 fp16 to sym_int4, 17 us of bytes: 190 us (behind a 123 us copy to fp32 and a zero fill) with a warp per block
+// and two elements a lane; 43 us with 16-byte accesses, an element's scale search, conversion and shift one by one, and warps
+// that took two or three tiles each; 33 now (the L2 written over before).
 template <typename T, int KIND>
 __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ src, uint8_t* __restrict__ dst, int64_t rows,
-                                                       int64_t cols, int64_t ld, bool vec) {
+                                                       int64_t cols, int64_t ld, int wide, bool wide_dst) {
   constexpr bool k4 = KIND <= Q_FP4;
   __shared__ float table[16];
+  __shared__ Buckets buckets;
   if (KIND == Q_NF4 || KIND == Q_FP4) {
     if (threadIdx.x < 16) table[threadIdx.x] = KIND == Q_NF4 ? c_nf4[threadIdx.x] : c_fp4[threadIdx.x & 7];
     __syncthreads();
+    if (KIND == Q_NF4) {
+      buckets.fill(table);
+      __syncthreads();
+    }
   }
   const int lane = threadIdx.x & 31, rr = lane >> 1, half = lane & 1;
   const int64_t Np = ceil_to_i64(rows, 16), Kp = ceil_to_i64(cols, 128);
@@ -95,33 +192,21 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ src
     const bool valid = r < rows && k0 < cols;
     Run64<T> v;
     if (valid) {
-      v.load(src + r * ld + k0, vec);
+      v.load(src + r * ld + k0, wide);
     } else {
 #pragma unroll
       for (int i = 0; i < Run64<T>::kWords; ++i) v.w[i] = 0;
     }
     if constexpr (k4) {
-      float d, mn = 0.f;
+      float d, mn, hi;
+      v.extremes(mn, hi);
       if (KIND == Q_ASYM4) {
-        float lo = v.at(0), hi = lo;
-#pragma unroll
-        for (int i = 1; i < 64; ++i) {
-          lo = fminf(lo, v.at(i));
-          hi = fmaxf(hi, v.at(i));
-        }
-        d = __fdiv_rn(__fsub_rn(hi, lo), 15.0f);
-        mn = lo;
+        d = __fdiv_rn(__fsub_rn(hi, mn), 15.0f);
       } else {
-        // the first of the largest magnitudes, as the serial host loop finds it
-        float top = v.at(0), best = fabsf(top);
-#pragma unroll
-        for (int i = 1; i < 64; ++i) {
-          const float x = v.at(i), m = fabsf(x);
-          if (m > best) { best = m; top = x; }
-        }
+        const float top = v.first_largest(mn, hi);
         if (KIND == Q_SYM4) d = __fdiv_rn(top, -8.0f);
-        else if (KIND == Q_NF4) d = best;
-        else d = __fdiv_rn(best, 6.0f);
+        else if (KIND == Q_NF4) d = fabsf(top);
+        else d = __fdiv_rn(fabsf(top), 6.0f);
       }
       const __half dh = __float2half_rn(d);
       const float ds = (KIND == Q_SYM4 || KIND == Q_ASYM4) ? d : __half2float(dh);
@@ -129,22 +214,20 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ src
       uint32_t w[8];
 #pragma unroll
       for (int o = 0; o < 8; ++o) {
-        w[o] = 0;
+        if (KIND == Q_SYM4 || KIND == Q_ASYM4) {
+          // nibble of element k: {0, 4, 1, 5, 2, 6, 3, 7}
+          w[o] = nibbles([&](int n) {
+            const float x = v.at(8 * o + 2 * (n & 3) + (n >> 2));
+            return KIND == Q_SYM4 ? __fadd_rn(__fmul_rn(x, id), 8.5f) : __fadd_rn(__fmul_rn(__fsub_rn(x, mn), id), 0.5f);
+          });
+        } else {
+          w[o] = 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float x = v.at(8 * o + k);
-          int q;
-          if (KIND == Q_SYM4) {
-            q = min(15, max(0, (int)__fadd_rn(__fmul_rn(x, id), 8.5f)));
-          } else if (KIND == Q_ASYM4) {
-            q = min(15, max(0, (int)__fadd_rn(__fmul_rn(__fsub_rn(x, mn), id), 0.5f)));
-          } else {
-            const float sx = __fmul_rn(x, id);
-            q = KIND == Q_NF4 ? nearest_sorted<16>(table, sx) : (nearest_sorted<8>(table, fabsf(sx)) | (sx < 0.f ? 8 : 0));
+          for (int k = 0; k < 8; ++k) {
+            const float sx = __fmul_rn(v.at(8 * o + k), id);
+            const int q = KIND == Q_NF4 ? buckets.nearest(sx) : (nearest_sorted<8>(table, fabsf(sx)) | (sx < 0.f ? 8 : 0));
+            w[o] |= (uint32_t)q << (4 * k);
           }
-          // nibble of element k: {0, 4, 1, 5, 2, 6, 3, 7} in the integer formats, k in the code books
-          const int slot = (KIND == Q_SYM4 || KIND == Q_ASYM4) ? (k >> 1) + 4 * (k & 1) : k;
-          w[o] |= (uint32_t)q << (4 * slot);
         }
         if (!valid) w[o] = 0;
       }
@@ -152,41 +235,42 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ src
       uint32_t got[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) got[i] = __shfl_xor_sync(0xffffffffu, half ? w[i] : w[4 + i], 1);
-      uint4* out = reinterpret_cast<uint4*>(dst + tile * 1024 + rr * 64 + half * 32);
-      if (half == 0) {
-        out[0] = make_uint4(w[0], w[1], got[0], got[1]);
-        out[1] = make_uint4(w[2], w[3], got[2], got[3]);
-      } else {
-        out[0] = make_uint4(got[0], got[1], w[4], w[5]);
-        out[1] = make_uint4(got[2], got[3], w[6], w[7]);
-      }
+      uint8_t* to = dst + tile * 1024 + rr * 64 + half * 32;
+      if (half == 0) store32(to, make_uint4(w[0], w[1], got[0], got[1]), make_uint4(w[2], w[3], got[2], got[3]), wide_dst);
+      else store32(to, make_uint4(got[0], got[1], w[4], w[5]), make_uint4(got[2], got[3], w[6], w[7]), wide_dst);
       const int64_t si = (tile * 2 + half) * 16 + pair_row(rr);
       sc16[si] = valid ? __half_as_ushort(dh) : (uint16_t)0;
       if (KIND == Q_ASYM4) (sc16 + Np * (Kp / 64))[si] = valid ? __half_as_ushort(__float2half_rn(mn)) : (uint16_t)0;
     } else {
-      float amax = 0.f;
-#pragma unroll
-      for (int i = 0; i < 64; ++i) amax = fmaxf(amax, fabsf(v.at(i)));
+      float lo, hi;
+      v.extremes(lo, hi);
+      float amax = fmaxf(0.f, fmaxf(-lo, hi));
       if (KIND != Q_INT8) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
       const float d = __fdiv_rn(amax, KIND == Q_INT8 ? 127.0f : KIND == Q_E4M3 ? 448.0f : 57344.0f);
       const float id = d != 0.f ? __fdiv_rn(1.0f, d) : 0.f;
       uint32_t w[16];
 #pragma unroll
       for (int o = 0; o < 16; ++o) {
-        w[o] = 0;
+        float sx[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float sx = __fmul_rn(v.at(4 * o + k), id);
-          uint32_t c;
-          if (KIND == Q_INT8) c = (uint8_t)(int8_t)min(127, max(-128, __float2int_rn(sx)));
-          else c = (uint8_t)__nv_cvt_float_to_fp8(sx, __NV_SATFINITE, KIND == Q_E4M3 ? __NV_E4M3 : __NV_E5M2);
-          w[o] |= c << (8 * k);
+        for (int k = 0; k < 4; ++k) sx[k] = __fmul_rn(v.at(4 * o + k), id);
+        if (KIND == Q_INT8) {
+          w[o] = 0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            w[o] |= (uint32_t)(uint8_t)(int8_t)min(127, max(-128, __float2int_rn(sx[k]))) << (8 * k);
+        } else {
+          constexpr auto kFp8 = KIND == Q_E4M3 ? __NV_E4M3 : __NV_E5M2;
+          w[o] = (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(sx[0], sx[1]), __NV_SATFINITE, kFp8) |
+                 (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(sx[2], sx[3]), __NV_SATFINITE, kFp8) << 16;
         }
         if (!valid) w[o] = 0;
       }
-      uint4* out = reinterpret_cast<uint4*>(dst + (tile * 2 + half) * 1024 + rr * 64);
+      uint8_t* to = dst + (tile * 2 + half) * 1024 + rr * 64;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) out[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+      for (int i = 0; i < 2; ++i)
+        store32(to + 32 * i, make_uint4(w[8 * i], w[8 * i + 1], w[8 * i + 2], w[8 * i + 3]),
+                make_uint4(w[8 * i + 4], w[8 * i + 5], w[8 * i + 6], w[8 * i + 7]), wide_dst);
       if (KIND == Q_INT8) {
         sc16[(tile * 2 + half) * 16 + pair_row(rr)] = valid ? __half_as_ushort(__float2half_rn(d)) : (uint16_t)0;
       } else if (half == 0) {
@@ -501,22 +585,24 @@ IPEX_API int ipex_quantize_to_tiles(const void* src, void* dst, int64_t rows, in
   if (rows < 1 || cols < 1) return (int)cudaSuccess;
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t work = ceil_to_i64(rows, 16) / 16 * (ceil_to_i64(cols, 128) / 128);
-  const int blocks = (int)(work + 7 < 8 * 148 * 8 ? (work + 7) / 8 : 148 * 8);
+  const int blocks = (int)((work + 7) / 8 < 148 * 64 ? (work + 7) / 8 : 148 * 64);    // a tile to a warp: no last round
   return by_dtype3(dtype, [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
     const T* p = (const T*)src;
     uint8_t* d = (uint8_t*)dst;
-    const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (ld * sizeof(T)) % 16 == 0;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(src) | (uintptr_t)(ld * sizeof(T));
+    const int wide = (at & 31) == 0 ? 32 : (at & 15) == 0 ? 16 : 1;
+    const bool whole = (reinterpret_cast<uintptr_t>(dst) & 31) == 0;
     switch (wf) {
-      case WF_SYM_INT4: quantize_kernel<T, Q_SYM4><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, vec); break;
-      case WF_ASYM_INT4: quantize_kernel<T, Q_ASYM4><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, vec); break;
+      case WF_SYM_INT4: quantize_kernel<T, Q_SYM4><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, wide, whole); break;
+      case WF_ASYM_INT4: quantize_kernel<T, Q_ASYM4><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, wide, whole); break;
       case WF_LUT4:
-        if (lut_kind == 0) quantize_kernel<T, Q_NF4><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, vec);
-        else quantize_kernel<T, Q_FP4><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, vec);
+        if (lut_kind == 0) quantize_kernel<T, Q_NF4><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, wide, whole);
+        else quantize_kernel<T, Q_FP4><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, wide, whole);
         break;
-      case WF_FP8_E4M3: quantize_kernel<T, Q_E4M3><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, vec); break;
-      case WF_FP8_E5M2: quantize_kernel<T, Q_E5M2><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, vec); break;
-      case WF_INT8: quantize_kernel<T, Q_INT8><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, vec); break;
+      case WF_FP8_E4M3: quantize_kernel<T, Q_E4M3><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, wide, whole); break;
+      case WF_FP8_E5M2: quantize_kernel<T, Q_E5M2><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, wide, whole); break;
+      case WF_INT8: quantize_kernel<T, Q_INT8><<<blocks, 256, 0, s>>>(p, d, rows, cols, ld, wide, whole); break;
       default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -527,7 +613,7 @@ IPEX_API int ipex_dequantize_tiles(const void* w, void* out, int64_t rows, int64
                                    const float* lut, int dtype, void* stream) {
   if (rows < 1 || cols < 1) return (int)cudaSuccess;
   const int64_t work = ceil_to_i64(rows, 16) / 16 * (ceil_to_i64(cols, 128) / 128);
-  const int blocks = (int)(work + 7 < 8 * 148 * 8 ? (work + 7) / 8 : 148 * 8);
+  const int blocks = (int)((work + 7) / 8 < 148 * 64 ? (work + 7) / 8 : 148 * 64);
   return by_dtype3(dtype, [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
     const uintptr_t at = reinterpret_cast<uintptr_t>(out) | (uintptr_t)(ld * sizeof(T));

@@ -75,3 +75,31 @@ def test_expand_into_rows_of_any_alignment(name, dtype):
         rc = cuda_lib().ipex_dequantize_tiles(ptr(packed), ptr(buf), N, K, K + gap, QTYPE_TO_WF[q], None, api.dtype_code(dtype),
                                               current_stream())
         assert rc == 0 and torch.equal(buf[:, :K], dense) and bool((buf[:, K:] == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("name", ["sym_int4", "asym_int4", "nf4", "fp4", "sym_int8"])
+def test_blocks_whose_scale_or_code_is_a_close_call(name, dtype):
+    """Largest values of both signs in either order, zeros of either sign, elements on and between the values of a code book."""
+    from ipex_llm_b200.ops.cuda_ops import dequantize_device
+    from ipex_llm_b200.ops.cuda_quant import quantize_to_device_layout
+    from ipex_llm_b200.quant import qtypes as qt
+    from ipex_llm_b200.quant.params import ggml_convert_fp32, ggml_convert_qtype
+    q = qt.qtype_from_name(name)
+    w = torch.randn(24, 128, generator=torch.Generator().manual_seed(2)) * 0.1
+    w[0, 5], w[0, 9], w[1, 5], w[1, 9] = 0.5, -0.5, -0.5, 0.5
+    w[2, 0], w[2, 63], w[3, 0], w[3, 63] = -2.0, 2.0, 2.0, -2.0
+    w[4], w[5], w[5, 1::2] = 0.0, 0.0, -0.0
+    w[6] = torch.where(torch.arange(128) % 2 == 0, -1.0, 1.0)
+    from ipex_llm_b200.ops.cuda_ops import _FP4, _NF4
+    for row, book in ((7, _NF4), (8, [v / 6 for v in _FP4])):
+        book = torch.tensor(sorted(book))
+        w[row, :16], w[row, 16:31], w[row, 64], w[row, 65:81] = book, (book[1:] + book[:-1]) / 2, 1.0, book * (1 + 2.0 ** -9)
+        w[row, 0] = 1.0
+    w[9:] = (w[9:] * 30).round() / 8                          # many equal magnitudes
+    w = w.to(dtype)
+    packed = quantize_to_device_layout(w.cuda(), q)
+    host = ggml_convert_fp32(ggml_convert_qtype(w.float().contiguous(), q).view(torch.uint8), w.shape, w.numel(), q)
+    assert torch.equal(dequantize_device(packed, w.shape, q, torch.float32).cpu(), host)
+    room = torch.empty(packed.numel() + 16, dtype=torch.uint8, device="cuda")
+    assert torch.equal(quantize_to_device_layout(w.cuda(), q, out=room[16:]), packed)
