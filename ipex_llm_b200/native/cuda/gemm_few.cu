@@ -1,10 +1,8 @@
 // Entry of the product for few rows and its fp16 instances (gemm_few.cuh).
 #include "gemm_few.cuh"
 
-// gemm_few_tcgen05.cu: the same through expanded weights in shared memory.
-IPEX_API int ipex_gemm_few_tcgen05(const void* x, const void* w, void* out, const void* bias, const void* residual,
-                                   const float* lut, int M, int N, int K, int64_t ldx, int64_t ldo, int64_t ldr, int wf,
-                                   int act, int pairs, int dtype, int pdl, int* err, void* stream);
+// gemm_few_tcgen05.cu
+int gemm_few_tcgen05(int wf, int dtype, const few::Operands& o, const few::Args& a, cudaStream_t st, bool pdl, int split);
 int gemm_few_bf16(int wf, const few::Operands& o, const few::Args& a, cudaStream_t st, bool pdl, int split);
 
 // out[M, N] = x . W^T (+ bias) (+ residual), or act(gate) * up with N / 2 columns, packed `w` of family `wf`, M <= 64 (32 with
@@ -22,11 +20,6 @@ IPEX_API int ipex_gemm_few(const void* x, const void* w, void* out, const void* 
   if (act != 0 && (residual != nullptr || (N % 32) != 0)) return (int)cudaErrorInvalidValue;
   if (wf == WF_LUT4 && lut == nullptr) return (int)cudaErrorInvalidValue;
   if ((wf == WF_FP8_E4M3 || wf == WF_FP8_E5M2) && (K % 128) != 0) return (int)cudaErrorInvalidValue;
-  // More than 48 rows of 4-bit integers, which that form expands and scales in 16 bits: 64 rows, 22016 x 4096 55.5 us there and
-  // 59 here, 12288 x 4096 31 and 36; at 48 rows 55 and 49.
-  if (rows > 48 && !pairs && split == 0 && K % 128 == 0 && (wf == WF_SYM_INT4 || wf == WF_ASYM_INT4) &&
-      (reinterpret_cast<uintptr_t>(w) & 31) == 0)
-    return ipex_gemm_few_tcgen05(x, w, out, bias, residual, lut, M, N, K, ldx, ldo, ldr, wf, act, 0, dtype, pdl, err, stream);
   const few::Operands o = {reinterpret_cast<const uint8_t*>(w), x, ldx, N, K};
   few::Args a = {};
   a.lut = lut;
@@ -38,5 +31,10 @@ IPEX_API int ipex_gemm_few(const void* x, const void* w, void* out, const void* 
   a.pairs = pairs;
   a.err = err;
   cudaStream_t st = (cudaStream_t)stream;
+  // From 25 rows on the weights' operand in tensor memory is the faster way (figures there); two rows to a token, or minima, keep
+  // the codes apart from their scales, which it does up to 32 columns or where a stage has one scale.
+  const bool fp8 = wf == WF_FP8_E4M3 || wf == WF_FP8_E5M2;
+  if (rows > 24 && (rows <= 32 ? wf != WF_ASYM_INT4 : !pairs || fp8))
+    return gemm_few_tcgen05(wf, dtype, o, a, st, pdl != 0, split);
   return dtype == DT_F16 ? few::by_family<__half>(wf, o, a, st, pdl != 0, split) : gemm_few_bf16(wf, o, a, st, pdl != 0, split);
 }

@@ -1,4 +1,5 @@
-// Products of 1 to 64 token rows with packed weights (decode steps of a batch, drafted continuations):
+// Products of 1 to 64 token rows with packed weights (decode steps of a batch, drafted continuations), most of those with up to
+// 24 rows by this kernel, the others by gemm_few_tcgen05.cuh:
 //     out[M, N] = x[M, K] . W[N, K]^T  (+ bias) (+ residual)   or   act(gate) * up  for interleaved gate/up rows
 //
 // What bounds it: with so few rows the weights' codes have to be taken apart as fast as they arrive, some nine instructions
@@ -17,11 +18,10 @@
 // a fixed order.  One warp fills the ring: the weights' part of the first stages is asked for before the kernel in front has
 // ended.
 //
-// Measured (us per launch between dependent launches, weights from memory; the tcgen05 form that wrote expanded weights to
-// shared memory -> this one): int4, 32 rows, 12288 x 4096 22.8 -> 21.5, 22016 x 4096 42.5 -> 33.7, 32000 x 4096 50.1 -> 37.0;
-// 16 rows 19.4 -> 14.6, 32.5 -> 22.1, 39.7 -> 23.6; fp8 and nf4, 40 rows, 22016 x 4096 64 and 67 -> 48.  ncu, 32000 x 4096 at 8
-// rows: half of the issue slots are used, 340 instructions for 4096 weights of which 150 take codes apart; at 32 rows the
-// matrix pipe (one m16n8k16 in 8 clocks) and the issue share the blame.
+// Measured (us per launch between dependent launches, weights from memory; a tcgen05 form that wrote expanded weights to shared
+// memory -> this one): int4, 16 rows, 12288 x 4096 19.4 -> 14.6, 22016 x 4096 32.5 -> 22.1, 32000 x 4096 39.7 -> 23.6.  ncu, 32000
+// x 4096 at 8 rows: half of the issue slots are used, 340 instructions for 4096 weights of which 150 take codes apart; from 24
+// rows on the matrix pipe (one m16n8k16 in 8 clocks) and the sums cost as much again: gemm_few_tcgen05.cuh.
 //
 // x may hold two rows per token (2m: the value rounded to 16 bits, 2m + 1: what that left over); their products are added in
 // 32 bits at the end.
@@ -113,13 +113,20 @@ __device__ __forceinline__ void mma16(float (&c)[4], uint32_t a0, uint32_t a1, u
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// The codes of 8 consecutive weights of a row as 16-bit values, in pairs of consecutive k.
+// The codes of 8 consecutive weights of a row as 16-bit values (not CODES: the weights), in pairs of consecutive k.
 template <typename T, int WF, bool CODES>
 __device__ __forceinline__ uint4 codes4(uint32_t w, const uint32_t* book, const Scale<T>& sc) {
   using V = V2<T>;
   constexpr float zero = WF == WF_SYM_INT4 ? 8.f : 0.f;
   if constexpr (WF == WF_LUT4) {       // `book` is this lane's copy
-    return make_uint4(book[(w & 0xFF) * 32], book[((w >> 8) & 0xFF) * 32], book[((w >> 16) & 0xFF) * 32], book[(w >> 24) * 32]);
+    uint4 v = make_uint4(book[(w & 0xFF) * 32], book[((w >> 8) & 0xFF) * 32], book[((w >> 16) & 0xFF) * 32], book[(w >> 24) * 32]);
+    if constexpr (!CODES) {
+      v.x = V::raw(__hmul2(V::bits(v.x), sc.d));
+      v.y = V::raw(__hmul2(V::bits(v.y), sc.d));
+      v.z = V::raw(__hmul2(V::bits(v.z), sc.d));
+      v.w = V::raw(__hmul2(V::bits(v.w), sc.d));
+    }
+    return v;
   } else if constexpr (!CODES) {
     return expand4<T, WF>(w, sc, nullptr);
   } else if constexpr (std::is_same<T, __half>::value) {
@@ -269,6 +276,67 @@ __device__ __forceinline__ void chunk_mma(const uint8_t* ct, const uint8_t* st, 
   }
 }
 
+// The code book: a pair of values by the byte, a copy for each lane, so that no two meet in a bank (eight copies: 22016 x 4096 at
+// 64 rows 41 -> 51 us).
+template <typename T> __device__ __forceinline__ void fill_book(uint32_t* book, const float* lut) {
+  for (int i = threadIdx.x; i < 256 * 8; i += kThreads) {
+    const int e = i >> 3;
+    const T lo = from_float<T>(lut[e & 15]), hi = from_float<T>(lut[e >> 4]);
+    const uint32_t v = (uint32_t)(*reinterpret_cast<const uint16_t*>(&lo)) |
+                       ((uint32_t)(*reinterpret_cast<const uint16_t*>(&hi)) << 16);
+    reinterpret_cast<uint4*>(book)[i] = make_uint4(v, v, v, v);
+  }
+}
+
+// The parts of a tile, PARTS of them [COLS][rows] in `red` of every CTA that shares it: a warp adds up 32 rows of one token at a
+// time, bias, residual or activation included.
+template <typename T, int PARTS, int COLS>
+__device__ __forceinline__ void add_parts(const Args& a, const float* red, int rank, int split, int tile, int warp, int lane) {
+  constexpr int kPitch = kBM + 4;
+  __syncthreads();
+  if (split > 1) cluster_sync_all();
+  {
+    pdl_wait();                                     // out and residual belong to the kernels before this one until here
+    const T* res = reinterpret_cast<const T*>(a.residual);
+    const T* bias = reinterpret_cast<const T*>(a.bias);
+    T* out = reinterpret_cast<T*>(a.out);
+    const uint32_t base = smem_u32(red);
+    for (int item = rank * kWarps + warp; item < 4 * a.M; item += split * kWarps) {
+      const int u = item & 3, m = item >> 2, n = tile * kBM + u * 32 + lane;
+      if (tile * kBM + u * 32 >= a.N) continue;
+      const int col = a.pairs ? 2 * m : m;
+      const uint32_t off = (uint32_t)((col * kPitch + u * 32 + lane) * 4);
+      float f = 0.f, v[kMaxSplit][PARTS], v2[kMaxSplit][PARTS];
+#pragma unroll
+      for (int q = 0; q < kMaxSplit; ++q) {
+        if (q >= split) break;
+        const uint32_t from = (split > 1 ? at_rank(base, q) : base) + off;
+#pragma unroll
+        for (int k = 0; k < PARTS; ++k) {
+          v[q][k] = ld_rank(from + k * COLS * kPitch * 4);
+          v2[q][k] = a.pairs ? ld_rank(from + (k * COLS + 1) * kPitch * 4) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kMaxSplit; ++q) {
+        if (q >= split) break;
+#pragma unroll
+        for (int k = 0; k < PARTS; ++k) f += v[q][k] + v2[q][k];
+      }
+      if (bias != nullptr && n < a.N) f += to_float(bias[n]);
+      if (a.act != 0) {
+        const float up = __shfl_down_sync(0xffffffffu, f, 16);
+        const int no = (tile * kBM + u * 32) / 2 + lane;
+        if (lane < 16 && no < a.N / 2) out[(int64_t)m * a.ldo + no] = from_float<T>(act_apply(f, a.act) * up);
+      } else if (n < a.N) {
+        if (res != nullptr) f += to_float(res[(int64_t)m * a.ldr + n]);
+        out[(int64_t)m * a.ldo + n] = from_float<T>(f);
+      }
+    }
+  }
+  if (split > 1) cluster_sync_all();                // no CTA leaves while another may still read its part
+}
+
 template <typename T, int WF, int NT, int WN>
 __global__ void __launch_bounds__(kThreads, kCtasPerSM)
 kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_x,
@@ -313,15 +381,7 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
     __syncwarp();
     for (int i = 0; i < S && i < nst; ++i) load_weights(i, i);
   }
-  if constexpr (WF == WF_LUT4) {
-    for (int i = threadIdx.x; i < 256 * 8; i += kThreads) {
-      const int e = i >> 3;
-      const T lo = from_float<T>(a.lut[e & 15]), hi = from_float<T>(a.lut[e >> 4]);
-      const uint32_t v = (uint32_t)(*reinterpret_cast<const uint16_t*>(&lo)) |
-                         ((uint32_t)(*reinterpret_cast<const uint16_t*>(&hi)) << 16);
-      reinterpret_cast<uint4*>(book)[i] = make_uint4(v, v, v, v);
-    }
-  }
+  if constexpr (WF == WF_LUT4) fill_book<T>(book, a.lut);
   __syncthreads();
   pdl_launch_dependents();
   if (warp == 0) {
@@ -374,49 +434,7 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
 #pragma unroll
         for (int i = 0; i < 4; ++i) mine[(n * 8 + 2 * t + (i & 1)) * C::kRedPitch + m * 16 + g + 8 * (i >> 1)] = acc[m][n][i];
   }
-  // ---------------- the parts of the tile: a warp adds up 32 rows of one token at a time ----------------
-  __syncthreads();
-  if (split > 1) cluster_sync_all();
-  {
-    pdl_wait();                                     // out and residual belong to the kernels before this one until here
-    const T* res = reinterpret_cast<const T*>(a.residual);
-    const T* bias = reinterpret_cast<const T*>(a.bias);
-    T* out = reinterpret_cast<T*>(a.out);
-    const uint32_t base = smem_u32(red);
-    for (int item = rank * kWarps + warp; item < 4 * a.M; item += split * kWarps) {
-      const int u = item & 3, m = item >> 2, n = tile * kBM + u * 32 + lane;
-      if (tile * kBM + u * 32 >= a.N) continue;
-      const int col = a.pairs ? 2 * m : m;
-      const uint32_t off = (uint32_t)((col * C::kRedPitch + u * 32 + lane) * 4);
-      float f = 0.f, v[kMaxSplit][C::WK], v2[kMaxSplit][C::WK];
-#pragma unroll
-      for (int q = 0; q < kMaxSplit; ++q) {
-        if (q >= split) break;
-        const uint32_t from = (split > 1 ? at_rank(base, q) : base) + off;
-#pragma unroll
-        for (int k = 0; k < C::WK; ++k) {
-          v[q][k] = ld_rank(from + k * C::kCols * C::kRedPitch * 4);
-          v2[q][k] = a.pairs ? ld_rank(from + (k * C::kCols + 1) * C::kRedPitch * 4) : 0.f;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < kMaxSplit; ++q) {
-        if (q >= split) break;
-#pragma unroll
-        for (int k = 0; k < C::WK; ++k) f += v[q][k] + v2[q][k];
-      }
-      if (bias != nullptr && n < a.N) f += to_float(bias[n]);
-      if (a.act != 0) {
-        const float up = __shfl_down_sync(0xffffffffu, f, 16);
-        const int no = (tile * kBM + u * 32) / 2 + lane;
-        if (lane < 16 && no < a.N / 2) out[(int64_t)m * a.ldo + no] = from_float<T>(act_apply(f, a.act) * up);
-      } else if (n < a.N) {
-        if (res != nullptr) f += to_float(res[(int64_t)m * a.ldr + n]);
-        out[(int64_t)m * a.ldo + n] = from_float<T>(f);
-      }
-    }
-  }
-  if (split > 1) cluster_sync_all();                // no CTA leaves while another may still read its part
+  add_parts<T, C::WK, C::kCols>(a, red, rank, split, tile, warp, lane);
 }
 
 // CTAs that share a tile's k: twice as many, up to eight, while all of them still fit the chip at two per SM or nearly so (a
@@ -449,31 +467,27 @@ inline bool encode_3d(CUtensorMap* tm, CUtensorMapDataType dt, const void* base,
 
 constexpr int kBadMap = -1;          // the driver's encoder refused the operands
 
-template <typename T, int WF, int NT, int WN>
-int launch(const Operands& o, Args a, cudaStream_t st, bool pdl, int asked) {
-  using C = Cfg<WF, NT, WN>;
-  auto kern = kernel<T, WF, NT, WN>;
-  static SmemLimit limit;
-  cudaError_t e = limit((const void*)kern, C::kSmem);
+// Tensor maps and launch of a kernel whose stage is WK chunks.
+template <typename T, int CODES, int PLANES, int COLS, int WK, typename K>
+int launch_tiles(K kern, SmemLimit& limit, int smem, const Operands& o, const Args& a, cudaStream_t st, bool pdl) {
+  cudaError_t e = limit((const void*)kern, smem);
   if (e != cudaSuccess) return (int)e;
-  const int tiles = (o.N + kBM - 1) / kBM;
-  a.split = pick_split(tiles, (a.chunks + C::WK - 1) / C::WK, asked);
   // codes: [16-row tile][1024 bytes of a chunk][128 words]; planes of scales: [plane][16-row tile][chunk's 8 words]; tokens:
   // [64 k][row][k].  Whatever lies outside is read as zero.
-  const cuuint64_t rt = ceil_to_i64(o.N, 16) / 16, ch = a.chunks, pieces = ch * (C::kCodes / 1024);
+  const cuuint64_t rt = ceil_to_i64(o.N, 16) / 16, ch = a.chunks, pieces = ch * (CODES / 1024);
   CUtensorMap tw, ts, tx;
   if (!encode_3d(&tw, CU_TENSOR_MAP_DATA_TYPE_INT64, o.w, {128, pieces, rt}, {1024, pieces * 1024},
-                 {128, (cuuint32_t)(C::WK * C::kCodes / 1024), 8}, CU_TENSOR_MAP_SWIZZLE_NONE) ||
-      !encode_3d(&ts, CU_TENSOR_MAP_DATA_TYPE_INT64, o.w + rt * pieces * 1024, {ch * 8, rt, (cuuint64_t)C::kPlanes},
-                 {ch * 64, rt * ch * 64}, {C::WK * 8, 8, C::kPlanes}, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+                 {128, (cuuint32_t)(WK * CODES / 1024), 8}, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+      !encode_3d(&ts, CU_TENSOR_MAP_DATA_TYPE_INT64, o.w + rt * pieces * 1024, {ch * 8, rt, (cuuint64_t)PLANES},
+                 {ch * 64, rt * ch * 64}, {WK * 8, 8, PLANES}, CU_TENSOR_MAP_SWIZZLE_NONE) ||
       !encode_3d(&tx, std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, o.x,
-                 {64, (cuuint64_t)a.rows, (cuuint64_t)o.K / 64}, {(cuuint64_t)o.ldx * 2, 128}, {64, C::kCols, 2 * C::WK},
+                 {64, (cuuint64_t)a.rows, (cuuint64_t)o.K / 64}, {(cuuint64_t)o.ldx * 2, 128}, {64, COLS, 2 * WK},
                  CU_TENSOR_MAP_SWIZZLE_128B))
     return kBadMap;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles * a.split);
+  cfg.gridDim = dim3((o.N + kBM - 1) / kBM * a.split);
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = C::kSmem;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -484,6 +498,14 @@ int launch(const Operands& o, Args a, cudaStream_t st, bool pdl, int asked) {
   cfg.attrs = at;
   cfg.numAttrs = pdl ? 2 : 1;
   return (int)cudaLaunchKernelEx(&cfg, kern, tw, ts, tx, a);
+}
+
+template <typename T, int WF, int NT, int WN>
+int launch(const Operands& o, Args a, cudaStream_t st, bool pdl, int asked) {
+  using C = Cfg<WF, NT, WN>;
+  a.split = pick_split((o.N + kBM - 1) / kBM, (a.chunks + C::WK - 1) / C::WK, asked);
+  static SmemLimit limit;
+  return launch_tiles<T, C::kCodes, C::kPlanes, C::kCols, C::WK>(kernel<T, WF, NT, WN>, limit, C::kSmem, o, a, st, pdl);
 }
 
 template <typename T, int WF>

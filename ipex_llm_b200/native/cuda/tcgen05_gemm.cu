@@ -681,8 +681,8 @@ IPEX_API int ipex_gemm_lowbit_tcgen05(const void* x, const void* w, void* out, c
   if (wf < WF_SYM_INT4 || wf > WF_INT8) return (int)cudaErrorInvalidValue;
   if (const int pt = pair_tile(M, N, false, w))
     return ipex_gemm_pair_tcgen05(x, w, out, bias, residual, lut, M, N, K, ldx, 0, ldo, ldr, wf, act, dtype, pt, err, stream);
-  // up to 64 rows: int4 at 32 rows 12288 x 4096 41.7 -> 21.5 us, 4096 x 4096 38.6 -> 10.6, 22016 x 4096 84 -> 33.7, 4096 x
-  // 11008 97 -> 17.7
+  // up to 64 rows: int4 at 32 rows 12288 x 4096 41.7 -> 17.5 us, 4096 x 4096 38.6 -> 9.3, 22016 x 4096 84 -> 29.3, 4096 x
+  // 11008 97 -> 14.4
   if (M <= 64 && K % 128 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0)
     return ipex_gemm_few(x, w, out, bias, residual, lut, M, N, K, ldx, ldo, ldr, wf, act, 0, dtype, 0, 0, err, stream);
   const int bt = ipex_gemm_tcgen05_token_tile(M);

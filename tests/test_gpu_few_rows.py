@@ -292,3 +292,30 @@ def test_long_rows_between_dependent_launches(name, dtype, M, K):
     ref = x.double() @ w.t() + bias.double() + z[:, :N].double()
     top = x.double().abs().amax(1, keepdim=True) * w.abs().sum(1)
     assert bool(((moved.double() - ref).abs() <= top * 2.0 ** -10 + ref.abs() * U[dtype]).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("name", ["sym_int4", "asym_int4", "nf4", "fp8_e4m3", "fp8_e5m2", "sym_int8"])
+def test_wide_rows_through_long_rings(name, dtype):
+    """25 to 64 rows on both sides of their column counts, over more stages than a ring holds, many tiles at once, again and again."""
+    from ipex_llm_b200.ops import cuda_ops, tcgen05_gemm
+    g = torch.Generator(device="cuda").manual_seed(9)
+    N, K = 3088, 4224
+    q, packed, w = _weights(name, N, K, dtype, g)
+    for M in (24, 25, 32, 33, 48, 49, 64):
+        x = torch.randn(M, K, device="cuda", generator=g).to(dtype)
+        mag, ref = x.double().abs() @ w.abs().t(), x.double() @ w.t()
+        codes = M <= 32 or name.startswith("fp8")
+        roundings = (8 if name == "asym_int4" else 3) if not codes else 1 if name == "nf4" else 0
+        spread = x.double().abs().sum(1, keepdim=True) * 0.5 * K ** 0.5 * 2.0 ** -23 if name == "asym_int4" else 0.0
+        bound = mag * (roundings * U[dtype] + K * 2.0 ** -23) + spread + ref.abs() * U[dtype] + 1e-6
+        for split in (0, 1, 5):
+            first = None
+            for _ in range(6):
+                out = torch.full((M, N), float("nan"), dtype=dtype, device="cuda")
+                assert tcgen05_gemm.gemm_few(x, packed, N, K, out, cuda_ops.QTYPE_TO_WF[q], lut=cuda_ops.lut_for(q, x.device),
+                                             split=split, pdl=True)
+                first = out if first is None else first
+                assert torch.equal(out, first)
+            assert bool(((first.double() - ref).abs() <= bound).all())
+    cuda_ops.check_error_flag(x.device)
