@@ -47,6 +47,7 @@ struct AttnArgs {
   int window;      // sliding window (0 = off)
   float scale;     // softmax scale
   float softcap;   // 0 = off
+  bool vec;        // q rows and the rotary table may be read 16 bytes at a time: see whole_rows()
 };
 
 __device__ __forceinline__ uint8_t to_e5m2(float v) {
@@ -113,8 +114,10 @@ struct RawKV {
 // HIDES: some query may not see some cached key (a window, or several queries whose keys are in the cache already).  Only then
 // a row asks for each key: the questions cost 5 - 12 % of a walk (32 sequences x 32 heads of 2048 fp16 tokens 197 us with
 // them and 184 without; 8 query heads to each of 8 kv heads, 2048 e5m2 tokens in 12 splits 36.6 and 33.0).
+// One row a warp of heads of 128 is held to four CTAs per SM, 128 registers (168 leave three; fp16: 32 sequences x 32 heads of 256
+// tokens 34.7 -> 30.4 us, 16 x 1024 63 -> 47.5).
 template <typename T, bool FP8, int D, int RW, bool HIDES>
-__global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
+__global__ void __launch_bounds__(kAttnThreads, RW == 1 && D == 128 ? 4 : 1) attn_decode_kernel(AttnArgs a) {
   constexpr int DPL = D / 8;
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -197,6 +200,39 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
       qpos[r] = i;
       const T* qp = reinterpret_cast<const T*>(a.q) + b * a.q_b + (int64_t)i * a.q_s + (int64_t)(kvh * G + gq) * a.q_h;
       const int pos = past + i;
+      if (a.vec) {
+        // The lane's elements, their partners half a head away and their rotary values are runs: some 16 requests instead of 64 of
+        // 2 and 4 bytes, which took the longer part of a short walk (32 sequences x 32 heads of 256 fp16 tokens 39.1 -> 34.7 us, one
+        // sequence x 32 heads of 1024 e5m2 tokens 11.0 -> 9.5 in four splits).
+        constexpr int half = D / 2;
+        const T* own = qp + ds * DPL;
+        const T* other = ds < 4 ? own + half : own - half;
+        const float* cr = a.cosp + (int64_t)pos * half + (ds & 3) * DPL;
+        const float* sr = a.sinp + (int64_t)pos * half + (ds & 3) * DPL;
+#pragma unroll
+        for (int d0 = 0; d0 < DPL; d0 += 8) {
+          const uint4 raw = *reinterpret_cast<const uint4*>(own + d0);
+          const T* x = reinterpret_cast<const T*>(&raw);
+          if (modeA && a.rope != 0) {
+            const uint4 raw2 = *reinterpret_cast<const uint4*>(other + d0);
+            const T* y = reinterpret_cast<const T*>(&raw2);
+            const float4 c4[2] = {*reinterpret_cast<const float4*>(cr + d0), *reinterpret_cast<const float4*>(cr + d0 + 4)};
+            const float4 s4[2] = {*reinterpret_cast<const float4*>(sr + d0), *reinterpret_cast<const float4*>(sr + d0 + 4)};
+            const float* c = reinterpret_cast<const float*>(c4);
+            const float* sn = reinterpret_cast<const float*>(s4);
+#pragma unroll
+            for (int d = 0; d < 8; d++) {
+              const float v = DT<T>::to_f(x[d]), o = DT<T>::to_f(y[d]);
+              const float rot = ds < 4 ? v * c[d] - o * sn[d] : v * c[d] + o * sn[d];
+              qr[r][d0 + d] = DT<T>::to_f(DT<T>::from_f(rot)) * a.scale;
+            }
+          } else {
+#pragma unroll
+            for (int d = 0; d < 8; d++) qr[r][d0 + d] = DT<T>::to_f(x[d]) * a.scale;
+          }
+        }
+        continue;
+      }
 #pragma unroll
       for (int d = 0; d < DPL; d++) {
         const int e = ds * DPL + d;
@@ -421,7 +457,9 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
 #pragma unroll
     for (int r = 0; r < RW; r++) {
 #pragma unroll
-      for (int d = 0; d < DPL; d++) part_acc[(warp * RW + r) * D + ds * DPL + d] = acc[r][d];
+      for (int d = 0; d < DPL; d += 4)
+        *reinterpret_cast<float4*>(&part_acc[(warp * RW + r) * D + ds * DPL + d]) =
+            make_float4(acc[r][d], acc[r][d + 1], acc[r][d + 2], acc[r][d + 3]);
       if (ds == 0) {
         part_ml[(warp * RW + r) * 2 + 0] = m[r];
         part_ml[(warp * RW + r) * 2 + 1] = l[r];
@@ -512,6 +550,14 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(AttnArgs a) {
     T* op = reinterpret_cast<T*>(a.out) + b * a.o_b + (int64_t)i * a.o_s + (int64_t)(kvh * G + gq) * a.o_h;
     op[e] = DT<T>::from_f(ll > 0.f ? av / ll : 0.f);
   }
+}
+
+// Whether q rows and the rotary table may be read 16 bytes at a time: aligned, and heads rotated whole by halves (or not at all).
+static bool whole_rows(const AttnArgs& a, int D) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(a.q) | (uintptr_t)(2 * (a.q_b | a.q_s | a.q_h));
+  if (at & 15) return false;
+  if (a.knew == nullptr || a.rope == 0) return true;
+  return a.rope == 1 && a.R == D && ((reinterpret_cast<uintptr_t>(a.cosp) | reinterpret_cast<uintptr_t>(a.sinp)) & 15) == 0;
 }
 
 // IPEX_LLM_ATTN_RW4=1: 5..8 query rows per kv head use four rows per warp (two row groups, the warps of a group
@@ -619,6 +665,7 @@ IPEX_API int ipex_attn_decode(const void* q, const void* knew, const void* vnew,
   const int rows_total = (Hq / Hkv) * Sq;
   a.nrb = (rows_total + kMaxRows - 1) / kMaxRows;
   a.rope = rope; a.R = R; a.causal = causal; a.window = window; a.scale = scale; a.softcap = softcap;
+  a.vec = whole_rows(a, D);
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == DT_F16) {
     return (int)(fp8_kv ? launch_d<__half, true>(D, a, s, pdl != 0) : launch_d<__half, false>(D, a, s, pdl != 0));

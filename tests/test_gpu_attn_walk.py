@@ -108,3 +108,19 @@ def test_splits_fit_the_gpu(monkeypatch):
                 n = cuda_ops.attn_splits(B, Hkv, S, rows, 128, False, torch.bfloat16)
                 per_sm = cuda_ops._attn_ctas_per_sm(128, rows, False, 1)
                 assert 1 <= n <= 128 and (n == 1 or n * B * Hkv * -(-rows // 16) <= 148 * per_sm and S // n >= 160)
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("heads", [(4, 4), (8, 1)])
+def test_queries_of_any_alignment(heads, D):
+    """q rows that begin at two bytes, or lie apart by an odd number of elements, are read one by one: the same results."""
+    from ipex_llm_b200.ops import cuda_ops
+    Hq, Hkv = heads
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q = torch.randn(2, Hq, 3, D, device="cuda", generator=g).half()
+    k, v = (torch.randn(2, Hkv, 77, D, device="cuda", generator=g).half() for _ in range(2))
+    want = cuda_ops.sdpa_decode(q, k, v, None, D ** -0.5, None, None)
+    moved = torch.empty(q.numel() + 1, dtype=q.dtype, device="cuda")[1:].view(q.shape).copy_(q)
+    apart = torch.empty(*q.shape[:3], D + 3, dtype=q.dtype, device="cuda")[..., :D].copy_(q)
+    for other in (moved, apart):
+        assert torch.equal(cuda_ops.sdpa_decode(other, k, v, None, D ** -0.5, None, None), want)
