@@ -296,7 +296,6 @@ __device__ __forceinline__ void add_parts(const Args& a, const float* red, int r
   __syncthreads();
   if (split > 1) cluster_sync_all();
   {
-    pdl_wait();                                     // out and residual belong to the kernels before this one until here
     const T* res = reinterpret_cast<const T*>(a.residual);
     const T* bias = reinterpret_cast<const T*>(a.bias);
     T* out = reinterpret_cast<T*>(a.out);
@@ -384,8 +383,10 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
   if constexpr (WF == WF_LUT4) fill_book<T>(book, a.lut);
   __syncthreads();
   pdl_launch_dependents();
+  // The tokens come from the kernels before this one, out and residual belong to them until here.  Every warp waits for them
+  // here: the bounded waits below then count this kernel's own copies only.
+  pdl_wait();
   if (warp == 0) {
-    pdl_wait();                                     // the tokens come from the kernel before this one
     for (int i = 0; i < S && i < nst; ++i) load_tokens(i, i);
   }
   {

@@ -139,8 +139,8 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
   __syncthreads();
   tcgen05_fence_after();
   pdl_launch_dependents();                          // (with this CTA's columns allocated: a kernel behind may want its own)
+  pdl_wait();                                       // the tokens come from the kernels before this one (see gemm_few.cuh)
   if (warp == 0) {
-    pdl_wait();                                     // the tokens come from the kernel before this one
     for (int i = 0; i < S && i < nst; ++i) load_tokens(i, i, 0);
   }
 

@@ -319,3 +319,55 @@ def test_wide_rows_through_long_rings(name, dtype):
                 assert torch.equal(out, first)
             assert bool(((first.double() - ref).abs() <= bound).all())
     cuda_ops.check_error_flag(x.device)
+
+
+# A kernel that lets its dependents start at once, ends `ns` later and only then leaves the tokens behind.
+LATE = r"""
+extern "C" __global__ void late(const uint4* from, uint4* to, int n, unsigned long long ns) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  unsigned long long t0, t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+  t = t0;
+  for (int i = 0; i < 1 << 22 && t - t0 < ns; ++i) {
+    __nanosleep(1000);
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  }
+  for (int i = threadIdx.x; i < n; i += blockDim.x) to[i] = from[i];
+}
+"""
+
+
+def _ok(result):
+    assert int(result[0]) == 0, result
+    return result[1] if len(result) > 1 else None
+
+
+@pytest.mark.parametrize("M", [8, 40])
+def test_kernel_in_front_may_take_its_time(M):
+    """The bounded waits (half a second) count the product's own copies, not how long the kernel in front still runs."""
+    import ctypes
+    from cuda.bindings import driver, nvrtc
+    from ipex_llm_b200.ops import cuda_ops, tcgen05_gemm
+    prog = _ok(nvrtc.nvrtcCreateProgram(LATE.encode(), b"late.cu", 0, [], []))
+    _ok(nvrtc.nvrtcCompileProgram(prog, 1, [b"--gpu-architecture=sm_100a"]))
+    cubin = bytes(_ok(nvrtc.nvrtcGetCUBINSize(prog)))
+    _ok(nvrtc.nvrtcGetCUBIN(prog, cubin))
+    g = torch.Generator(device="cuda").manual_seed(M)
+    N, K = 272, 1152
+    q, packed, w = _weights("sym_int4", N, K, torch.float16, g)
+    x = torch.randn(M, K, device="cuda", generator=g).half()
+    late, out = torch.zeros_like(x), torch.empty(M, N, dtype=torch.float16, device="cuda")
+    want = torch.empty_like(out)
+    wf = cuda_ops.QTYPE_TO_WF[q]
+    assert tcgen05_gemm.gemm_few(x, packed, N, K, want, wf)
+    torch.cuda.synchronize()
+    module = _ok(driver.cuModuleLoadData(cubin))
+    kernel = _ok(driver.cuModuleGetFunction(module, b"late"))
+    args = ((x.data_ptr(), late.data_ptr(), x.numel() // 8, 3_000_000_000),
+            (ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64))
+    _ok(driver.cuLaunchKernel(kernel, 1, 1, 1, 128, 1, 1, 0, torch.cuda.current_stream().cuda_stream, args, 0))
+    assert tcgen05_gemm.gemm_few(late, packed, N, K, out, wf, pdl=True)
+    torch.cuda.synchronize()
+    _ok(driver.cuModuleUnload(module))
+    cuda_ops.check_error_flag(x.device)
+    assert torch.equal(out, want)
