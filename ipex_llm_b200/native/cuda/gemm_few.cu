@@ -22,6 +22,7 @@ IPEX_API int ipex_gemm_few(const void* x, const void* w, void* out, const void* 
   if ((wf == WF_FP8_E4M3 || wf == WF_FP8_E5M2) && (K % 128) != 0) return (int)cudaErrorInvalidValue;
   const few::Operands o = {reinterpret_cast<const uint8_t*>(w), x, ldx, N, K};
   few::Args a = {};
+  a.w = o.w; a.x = x; a.ldx = ldx; a.K = K;
   a.lut = lut;
   a.out = out; a.bias = bias; a.residual = residual; a.ldo = ldo; a.ldr = ldr;
   a.M = M; a.N = N;

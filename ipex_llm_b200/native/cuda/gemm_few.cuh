@@ -47,6 +47,10 @@ constexpr int kSmemMax = 113 * 1024;   // of a CTA, so that two fit an SM
 constexpr int kMaxSplit = 8;
 
 struct Args {
+  const uint8_t* w;
+  const void* x;
+  int64_t ldx;
+  int K;
   const float* lut;
   void* out;
   const void* bias;
@@ -288,6 +292,36 @@ template <typename T> __device__ __forceinline__ void fill_book(uint32_t* book, 
   }
 }
 
+// Sums that are no number, of this CTA's k0 .. k1 of a format with minima, once more from the weights themselves: beside an
+// infinite token the codes' part and the minimum's are infinities of any signs, or a zero code's product with it, where the
+// weight's own product is an infinity of the weight's sign.  Only rows with such a token (or without a number) come here.
+template <typename T, int PARTS, int COLS>
+__device__ __noinline__ void add_up_again(const Args& a, float* red, int tile, int k0, int k1) {
+  constexpr int kPitch = kBM + 4;
+  const int row = threadIdx.x % kBM, n = tile * kBM + row;
+  if (n >= a.N) return;
+  const int64_t row_tiles = ceil_to_i64(a.N, 16) / 16;
+  const uint8_t* scales = a.w + row_tiles * a.chunks * 1024;
+  for (int c = threadIdx.x / kBM; c < a.rows; c += kThreads / kBM) {
+    float* sum = red + c * kPitch + row;
+    bool number = true;
+    for (int p = 0; p < PARTS; ++p) number = number && sum[p * COLS * kPitch] == sum[p * COLS * kPitch];
+    if (number) continue;
+    const T* x = reinterpret_cast<const T*>(a.x) + c * a.ldx;
+    float again = 0.f;
+    for (int k = k0; k < k1; ++k) {
+      const int64_t chunk = (n >> 4) * (int64_t)a.chunks + (k >> 7);
+      const int h = (k >> 6) & 1, e = k & 7;
+      const uint32_t word = *reinterpret_cast<const uint32_t*>(a.w + chunk * 1024 + (n & 15) * 64 + ((k & 63) >> 4) * 16 + h * 8 +
+                                                               ((k >> 3) & 1) * 4);
+      const __half* d = reinterpret_cast<const __half*>(scales + chunk * 64) + h * 16 + pair_row(n & 15);
+      const float m = __half2float(d[row_tiles * a.chunks * 32]);
+      again = fmaf(fmaf(__half2float(*d), (float)((word >> (4 * ((e >> 1) + 4 * (e & 1)))) & 15), m), to_float(x[k]), again);
+    }
+    for (int p = 0; p < PARTS; ++p) sum[p * COLS * kPitch] = p == 0 ? again : 0.f;
+  }
+}
+
 // The parts of a tile, PARTS of them [COLS][rows] in `red` of every CTA that shares it: a warp adds up 32 rows of one token at a
 // time, bias, residual or activation included.
 template <typename T, int PARTS, int COLS>
@@ -339,7 +373,7 @@ __device__ __forceinline__ void add_parts(const Args& a, const float* red, int r
 template <typename T, int WF, int NT, int WN>
 __global__ void __launch_bounds__(kThreads, kCtasPerSM)
 kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_x,
-       const Args a) {
+       const __grid_constant__ Args a) {
   using C = Cfg<WF, NT, WN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* ring = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
@@ -434,6 +468,17 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
       for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) mine[(n * 8 + 2 * t + (i & 1)) * C::kRedPitch + m * 16 + g + 8 * (i >> 1)] = acc[m][n][i];
+    if constexpr (C::minima) {
+      float zero = 0.f;
+#pragma unroll
+      for (int m = 0; m < C::MT; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) zero = fmaf(acc[m][n][i], 0.f, zero);
+      if (__syncthreads_or(zero != 0.f))
+        add_up_again<T, C::WK, C::kCols>(a, red, tile, st0 * C::WK * 128, min(a.K, (st0 + nst) * C::WK * 128));
+    }
   }
   add_parts<T, C::WK, C::kCols>(a, red, rank, split, tile, warp, lane);
 }

@@ -371,3 +371,35 @@ def test_kernel_in_front_may_take_its_time(M):
     _ok(driver.cuModuleUnload(module))
     cuda_ops.check_error_flag(x.device)
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M", [1, 8, 9, 17, 25, 32, 40])
+def test_infinite_tokens_of_a_format_with_minima(M, dtype):
+    """An infinite token times a weight is an infinity of the weight's sign, whatever its code and its block's minimum are; two of
+    both signs are no number; the other rows do not notice."""
+    from ipex_llm_b200.ops import cuda_ops, cuda_quant, tcgen05_gemm
+    from ipex_llm_b200.quant import qtypes as qt
+    g = torch.Generator(device="cuda").manual_seed(M)
+    N, K = 272, 832
+    q = qt.qtype_from_name("asym_int4")
+    # rows of one sign, away from zero: with 4 bits between them, no weight rounds to it
+    w = (1 + torch.rand(N, K, device="cuda", generator=g)) * torch.where(torch.arange(N, device="cuda") % 2 == 0, 1, -1)[:, None]
+    packed = cuda_quant.quantize_to_device_layout(w.to(dtype), q)
+    wd = cuda_ops.dequantize_device(packed, (N, K), q, torch.float32).double()
+    x = torch.randn(M, K, device="cuda", generator=g).to(dtype)
+    bad = x.clone()
+    bad[0, 700] = float("inf")
+    bad[M // 2, [3, 130]] = float("-inf")
+    if M > 2:
+        bad[M - 1, 5], bad[M - 1, 400] = float("inf"), float("-inf")
+    ref = bad.double() @ wd.t()
+    hit = torch.isinf(bad).any(1)
+    for split in (0, 1, 3):
+        out, clean = (torch.empty(M, N, dtype=dtype, device="cuda") for _ in range(2))
+        assert tcgen05_gemm.gemm_few(bad, packed, N, K, out, cuda_ops.QTYPE_TO_WF[q], split=split)
+        assert tcgen05_gemm.gemm_few(x, packed, N, K, clean, cuda_ops.QTYPE_TO_WF[q], split=split)
+        torch.cuda.synchronize()
+        cuda_ops.check_error_flag(x.device)
+        assert torch.equal(out[hit].double().nan_to_num(7.0, 9.0, -9.0), ref[hit].nan_to_num(7.0, 9.0, -9.0))
+        assert torch.equal(out[~hit], clean[~hit])
