@@ -296,27 +296,27 @@ template <typename T> __device__ __forceinline__ void fill_book(uint32_t* book, 
 // infinite token the codes' part and the minimum's are infinities of any signs, or a zero code's product with it, where the
 // weight's own product is an infinity of the weight's sign.  Only rows with such a token (or without a number) come here.
 template <typename T, int PARTS, int COLS>
-__device__ __noinline__ void add_up_again(const Args& a, float* red, int tile, int k0, int k1) {
+__device__ __noinline__ void add_up_again(const uint8_t* w, const T* x, int64_t ldx, int rows, int N, int chunks, float* red, int tile, int k0,
+                                          int k1) {
   constexpr int kPitch = kBM + 4;
   const int row = threadIdx.x % kBM, n = tile * kBM + row;
-  if (n >= a.N) return;
-  const int64_t row_tiles = ceil_to_i64(a.N, 16) / 16;
-  const uint8_t* scales = a.w + row_tiles * a.chunks * 1024;
-  for (int c = threadIdx.x / kBM; c < a.rows; c += kThreads / kBM) {
+  if (n >= N) return;
+  const int64_t row_tiles = ceil_to_i64(N, 16) / 16;
+  const uint8_t* scales = w + row_tiles * chunks * 1024;
+  for (int c = threadIdx.x / kBM; c < rows; c += kThreads / kBM) {
     float* sum = red + c * kPitch + row;
     bool number = true;
     for (int p = 0; p < PARTS; ++p) number = number && sum[p * COLS * kPitch] == sum[p * COLS * kPitch];
     if (number) continue;
-    const T* x = reinterpret_cast<const T*>(a.x) + c * a.ldx;
     float again = 0.f;
     for (int k = k0; k < k1; ++k) {
-      const int64_t chunk = (n >> 4) * (int64_t)a.chunks + (k >> 7);
+      const int64_t chunk = (n >> 4) * (int64_t)chunks + (k >> 7);
       const int h = (k >> 6) & 1, e = k & 7;
-      const uint32_t word = *reinterpret_cast<const uint32_t*>(a.w + chunk * 1024 + (n & 15) * 64 + ((k & 63) >> 4) * 16 + h * 8 +
+      const uint32_t word = *reinterpret_cast<const uint32_t*>(w + chunk * 1024 + (n & 15) * 64 + ((k & 63) >> 4) * 16 + h * 8 +
                                                                ((k >> 3) & 1) * 4);
       const __half* d = reinterpret_cast<const __half*>(scales + chunk * 64) + h * 16 + pair_row(n & 15);
-      const float m = __half2float(d[row_tiles * a.chunks * 32]);
-      again = fmaf(fmaf(__half2float(*d), (float)((word >> (4 * ((e >> 1) + 4 * (e & 1)))) & 15), m), to_float(x[k]), again);
+      const float m = __half2float(d[row_tiles * chunks * 32]);
+      again = fmaf(fmaf(__half2float(*d), (float)((word >> (4 * ((e >> 1) + 4 * (e & 1)))) & 15), m), to_float(x[c * ldx + k]), again);
     }
     for (int p = 0; p < PARTS; ++p) sum[p * COLS * kPitch] = p == 0 ? again : 0.f;
   }
@@ -373,7 +373,7 @@ __device__ __forceinline__ void add_parts(const Args& a, const float* red, int r
 template <typename T, int WF, int NT, int WN>
 __global__ void __launch_bounds__(kThreads, kCtasPerSM)
 kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_x,
-       const __grid_constant__ Args a) {
+       const Args a) {
   using C = Cfg<WF, NT, WN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* ring = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
@@ -477,7 +477,8 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
 #pragma unroll
           for (int i = 0; i < 4; ++i) zero = fmaf(acc[m][n][i], 0.f, zero);
       if (__syncthreads_or(zero != 0.f))
-        add_up_again<T, C::WK, C::kCols>(a, red, tile, st0 * C::WK * 128, min(a.K, (st0 + nst) * C::WK * 128));
+        add_up_again<T, C::WK, C::kCols>(a.w, reinterpret_cast<const T*>(a.x), a.ldx, a.rows, a.N, a.chunks, red, tile,
+                                         st0 * C::WK * 128, min(a.K, (st0 + nst) * C::WK * 128));
     }
   }
   add_parts<T, C::WK, C::kCols>(a, red, rank, split, tile, warp, lane);
