@@ -32,10 +32,10 @@ IPEX_API int ipex_gemm_few(const void* x, const void* w, void* out, const void* 
   a.pairs = pairs;
   a.err = err;
   cudaStream_t st = (cudaStream_t)stream;
-  // From 25 rows on the weights' operand in tensor memory is the faster way (figures there); two rows to a token, or minima, keep
-  // the codes apart from their scales, which it does up to 32 columns or where a stage has one scale.
+  // From 25 rows on (17 with minima) the weights' operand in tensor memory is the faster way (figures there); two rows to a token
+  // keep the codes apart from their scales, which it does up to 32 columns or where a stage has one scale.
   const bool fp8 = wf == WF_FP8_E4M3 || wf == WF_FP8_E5M2;
-  if (rows > 24 && (rows <= 32 ? wf != WF_ASYM_INT4 : !pairs || fp8))
+  if (rows > (wf == WF_ASYM_INT4 ? 16 : 24) && (rows <= 32 || !pairs || fp8))
     return gemm_few_tcgen05(wf, dtype, o, a, st, pdl != 0, split);
   return dtype == DT_F16 ? few::by_family<__half>(wf, o, a, st, pdl != 0, split) : gemm_few_bf16(wf, o, a, st, pdl != 0, split);
 }

@@ -1,4 +1,5 @@
-// Products of 25 to 64 token rows with packed weights on tcgen05, the weights' operand in tensor memory:
+// Products of 25 to 64 token rows (17 to 64 of the format with minima) with packed weights on tcgen05, the weights' operand in
+// tensor memory:
 //     out[M, N] = x[M, K] . W[N, K]^T  (+ bias) (+ residual)   or   act(gate) * up  for interleaved gate/up rows
 // (gemm_few.cuh has the contract, the tensor maps, the ring's layout and the adding up of the parts.)
 //
@@ -13,6 +14,13 @@
 // Up to 32 columns (and in the 8-bit float formats) the codes are multiplied and the sums of each scale group scaled and added
 // in 32 bits.  More columns of the other formats are expanded and scaled in 16 bits, as in the kernel for many rows, and the sums
 // stay in tensor memory.
+//
+// Minima up to 32 columns stay apart too: their part is their product with the sums of the tokens, which a team makes (eight
+// tokens a warp, products with ones) and adds while its products run: the sums of a stage behind its barrier, their product with
+// the minima behind the next one's.  Sums by gemm_few.cuh's way (every warp makes all of them) and this, us at 24 | 32 rows of
+// fp16: 12288 x 4096 24.8 / 22.7 | 32.3 / 23.5, 4096 x 11008 20.2 / 18.4 | 26.0 / 18.9, 22016 x 4096 36.5 / 35.4 | 47.8 / 36.9 (bf16
+// 46.9 / 38.4); weights expanded and scaled in 16 bits (in a form before these) took 22.3, 19.2 and 34.6 at 32 rows.  (The minima's
+// product at the end, as tf32, instead of stage by stage: 24.1, 20.4 and 38.4.)
 //
 // A CTA holds 128 weight rows over a share of k; two teams of four warps take its stages of 128 k in turn, and two CTAs fit an SM,
 // so that three teams work while one waits.  A team that has waited for its products knows its stage's slot to be free and has it
@@ -31,6 +39,7 @@ template <int WF, int N> struct Cfg {
   static constexpr bool k4 = WF == WF_SYM_INT4 || WF == WF_ASYM_INT4 || WF == WF_LUT4;
   static constexpr bool fp8 = WF == WF_FP8_E4M3 || WF == WF_FP8_E5M2;
   static constexpr bool codes = fp8 || N <= 32;
+  static constexpr bool minima = WF == WF_ASYM_INT4 && codes;
   static constexpr int groups = codes && !fp8 ? 2 : 1;                 // sums of a stage
   static constexpr int kCodes = k4 ? 1024 : 2048, kScales = 64;        // bytes of a 16-row tile's 128 k
   static constexpr int kPlanes = WF == WF_ASYM_INT4 ? 2 : 1;
@@ -40,13 +49,14 @@ template <int WF, int N> struct Cfg {
   static constexpr int kBytes = kScaleAt + kPlanes * 8 * kScales;
   static constexpr int kStageBytes = (kBytes + 1023) / 1024 * 1024;
   static constexpr int kBook = WF == WF_LUT4 ? 256 * 32 * 4 : 0;
-  static constexpr int kTail = 256 + kBook;
+  static constexpr int kSums = minima ? kTeams * 2 * 2 * N * 4 : 0;    // [team][stage in turn][group][token]
+  static constexpr int kTail = 256 + kBook + kSums;
   static constexpr int kRedPitch = kBM + 4;
   static constexpr int kRedBytes = kTeams * N * kRedPitch * 4;
   static constexpr int kStagesFit = (kSmemMax - 1024 - kTail) / kStageBytes;
   static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;
   static constexpr int kSmem = 1024 + kStages * kStageBytes + kTail;
-  static_assert(kStages > kTeams && kRedBytes <= kStages * kStageBytes && groups * N <= kTeamCols - 64, "ring");
+  static_assert(kStages > kTeams && kRedBytes <= kStages * kStageBytes && groups * N <= kTeamCols - 64 && (!minima || N == 32), "ring");
 };
 
 __device__ __forceinline__ void tmem_st_32(uint32_t taddr, const uint32_t (&v)[32]) {
@@ -88,6 +98,20 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t bde
       : "memory");
 }
 
+// Two sums at once: a0 += d * x0, a1 += d * x1.
+__device__ __forceinline__ void fma2(float& a0, float& a1, float d, float x0, float x1) {
+  asm("{\n"
+      ".reg .b64 a, d, x;\n"
+      "mov.b64 a, {%0, %1};\n"
+      "mov.b64 d, {%2, %2};\n"
+      "mov.b64 x, {%3, %4};\n"
+      "fma.rn.f32x2 a, d, x, a;\n"
+      "mov.b64 {%0, %1}, a;\n"
+      "}\n"
+      : "+f"(a0), "+f"(a1)
+      : "f"(d), "f"(x0), "f"(x1));
+}
+
 template <typename T, int WF, int N>
 __global__ void __launch_bounds__(kThreads, kCtasPerSM)
 kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_x,
@@ -101,6 +125,7 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + kTeams);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint32_t* book = reinterpret_cast<uint32_t*>(full) + 64;
+  float* sums = reinterpret_cast<float*>(book);
   float* red = reinterpret_cast<float*>(ring);      // [team][column][row], once the ring has been read
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -165,9 +190,28 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
       for (int j = 0; j < step; j += 16) tmem_ld_16(tD + lanes + c + j, v + j);
       tmem_ld_done(v);
 #pragma unroll
-      for (int j = 0; j < step; ++j) {
+      for (int j = 0; j < step; j += 2) {
         if (c + j >= cols) break;
-        acc[(c + j) % N] = fmaf(d[(c + j) / N], v[j], acc[(c + j) % N]);
+        if constexpr (C::minima) {
+          fma2(acc[(c + j) % N], acc[(c + j) % N + 1], d[(c + j) / N], v[j], v[j + 1]);
+        } else {
+          acc[(c + j) % N] = fmaf(d[(c + j) / N], v[j], acc[(c + j) % N]);
+          acc[(c + j) % N + 1] = fmaf(d[(c + j) / N], v[j + 1], acc[(c + j) % N + 1]);
+        }
+      }
+    }
+  };
+  int turn = 0;                                     // where the stage's sums go
+  float dm[2] = {0.f, 0.f};                         // minima of the stage whose sums are there next
+  auto add_minima = [&] {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float4* sx = reinterpret_cast<const float4*>(sums + ((team * 2 + (turn ^ 1)) * 2 + h) * N);
+#pragma unroll
+      for (int j = 0; j < N; j += 4) {
+        const float4 x = sx[j / 4];
+        fma2(acc[j], acc[j + 1], dm[h], x.x, x.y);
+        fma2(acc[j + 2], acc[j + 3], dm[h], x.z, x.w);
       }
     }
   };
@@ -238,6 +282,15 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
     }
     d[0] = dn[0];
     d[1] = dn[1];
+    uint4 xb[C::minima ? 4 : 1];
+    if constexpr (C::minima) {
+      const int g = lane >> 2, t = lane & 3;
+      if (ok) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          xb[i] = *reinterpret_cast<const uint4*>(st + C::kXAt + (i >> 1) * C::kPiece + qd * 1024 + g * 128 + (((2 * t + (i & 1)) ^ g) << 4));
+      }
+    }
     tcgen05_fence_before();
     asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(kThreads / kTeams) : "memory");
     if (issuer && ok) {
@@ -255,6 +308,25 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
       }
       __syncwarp();
     }
+    if constexpr (C::minima) {
+      if (ok) {
+        if (waiting) add_minima();
+        constexpr uint32_t one = std::is_same<T, __half>::value ? 0x3C003C00u : 0x3F803F80u;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int o = 0; o < 2; ++o) {
+            mma16<T>(s, one, one, one, one, xb[2 * h + o].x, xb[2 * h + o].y);
+            mma16<T>(s, one, one, one, one, xb[2 * h + o].z, xb[2 * h + o].w);
+          }
+          if (lane < 4) *reinterpret_cast<float2*>(sums + ((team * 2 + turn) * 2 + h) * N + 8 * qd + 2 * lane) = make_float2(s[0], s[1]);
+        }
+      }
+      dm[0] = mn[0];
+      dm[1] = mn[1];
+      turn ^= 1;
+    }
     waiting = true;
     last = slot;
     last_use = use;
@@ -262,6 +334,10 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
     if (slot >= S) { slot -= S; ++use; }
   }
   if (waiting) {
+    if constexpr (C::minima) {
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(kThreads / kTeams) : "memory");
+      add_minima();
+    }
     if (ok) ok = warp_wait(&done[team], dph, abort_flag);
     tcgen05_fence_after();
     if (ok) {
@@ -284,6 +360,14 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
   float* mine = red + (size_t)team * N * C::kRedPitch + qd * 32 + lane;
 #pragma unroll
   for (int j = 0; j < N; ++j) mine[j * C::kRedPitch] = acc[j];
+  if constexpr (C::minima) {
+    float zero = 0.f;
+#pragma unroll
+    for (int j = 0; j < N; ++j) zero = fmaf(acc[j], 0.f, zero);
+    if (__syncthreads_or(zero != 0.f))
+      add_up_again<T, kTeams, N>(a.w, reinterpret_cast<const T*>(a.x), a.ldx, a.rows, a.N, a.chunks, red, tile, st0 * 128,
+                                 min(a.K, (st0 + nst) * 128));
+  }
   add_parts<T, kTeams, N>(a, red, rank, split, tile, warp, lane);
   if (warp == 1) {
     tcgen05_fence_after();
@@ -301,9 +385,7 @@ int launch(const Operands& o, Args a, cudaStream_t st, bool pdl, int asked) {
 
 template <typename T, int WF>
 int by_width(const Operands& o, const Args& a, cudaStream_t st, bool pdl, int asked) {
-  if constexpr (WF != WF_ASYM_INT4) {
-    if (a.rows <= 32) return launch<T, WF, 32>(o, a, st, pdl, asked);
-  }
+  if (a.rows <= 32) return launch<T, WF, 32>(o, a, st, pdl, asked);
   if (a.rows <= 48) return launch<T, WF, 48>(o, a, st, pdl, asked);
   return launch<T, WF, 64>(o, a, st, pdl, asked);
 }

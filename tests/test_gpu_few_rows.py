@@ -403,3 +403,24 @@ def test_infinite_tokens_of_a_format_with_minima(M, dtype):
         cuda_ops.check_error_flag(x.device)
         assert torch.equal(out[hit].double().nan_to_num(7.0, 9.0, -9.0), ref[hit].nan_to_num(7.0, 9.0, -9.0))
         assert torch.equal(out[~hit], clean[~hit])
+
+
+@pytest.mark.parametrize("K", [128, 448, 12288, 12416])
+@pytest.mark.parametrize("M", [16, 17, 32])
+def test_minima_of_many_stages(M, K):
+    """Minima up to 32 rows are not rounded on either side of the row count from which their product is made at the end, and of
+    the number of stages that it has room for (96 of a CTA)."""
+    from ipex_llm_b200.ops import cuda_ops, tcgen05_gemm
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    N = 400
+    for dtype in (torch.float16, torch.bfloat16):
+        q, packed, w = _weights("asym_int4", N, K, dtype, g)
+        x = torch.randn(M, K, device="cuda", generator=g).to(dtype)
+        mag, ref = x.double().abs() @ w.abs().t(), x.double() @ w.t()
+        spread = x.double().abs().sum(1, keepdim=True) * 0.5 * K ** 0.5 * 2.0 ** -23
+        for split in (0, 1, 2):
+            out = torch.full((M, N), float("nan"), dtype=dtype, device="cuda")
+            assert tcgen05_gemm.gemm_few(x, packed, N, K, out, cuda_ops.QTYPE_TO_WF[q], split=split)
+            torch.cuda.synchronize()
+            assert bool(((out.double() - ref).abs() <= mag * K * 2.0 ** -23 + spread + ref.abs() * U[dtype] + 1e-6).all())
+    cuda_ops.check_error_flag(x.device)
