@@ -111,13 +111,26 @@ struct RawKV {
   }
 };
 
+// CTAs that an SM is asked to hold; 0 leaves the registers to the compiler's own bounds (64, 96, 128 or 168), 1 gives a thread up
+// to 255.  us, 0 / 1 unless said:
+// One row of 128: four, 128 registers, where that does not spill (fp16: 32 sequences x 32 heads of 256 tokens 31.0 with 0 and 28.5,
+// of 2048 182 and 165; e5m2, 8 x 517 tokens 14.5 and 13.8).  bf16 caches and hidden fp16 keys spill under it (2048 bf16 tokens 184
+// with 0 and 294, 1024 fp16 tokens with a window 104 and 120).
+// Heads of 64 wait for memory and want the warps: 32 x 32 heads of 1024 fp16 tokens 51.9 / 59.2, e5m2 34.4 / 38.5; 8 queries to each
+// of 8 x 32 heads 79.4 / 102.
+// Everything else is the faster for its registers, though an SM holds a CTA less: 32 x 8 heads of 128 with 4 rows, 1024 e5m2
+// tokens 47.9 / 44.9, bf16 68.8 / 64.3, 8 x 32 x 4 queries fp16 80.9 / 72.1; 8 x 16 heads of 256 33.5 / 30.9, e5m2 23.2 / 21.6.
+template <typename T, bool FP8, int D, int RW, bool HIDES> constexpr int min_ctas() {
+  if (D == 64) return 0;
+  if (D == 128 && RW == 1) return FP8 || (std::is_same<T, __half>::value && !HIDES) ? 4 : 0;
+  return 1;
+}
+
 // HIDES: some query may not see some cached key (a window, or several queries whose keys are in the cache already).  Only then
 // a row asks for each key: the questions cost 5 - 12 % of a walk (32 sequences x 32 heads of 2048 fp16 tokens 197 us with
 // them and 184 without; 8 query heads to each of 8 kv heads, 2048 e5m2 tokens in 12 splits 36.6 and 33.0).
-// One row a warp of heads of 128 is held to four CTAs per SM, 128 registers (168 leave three; fp16: 32 sequences x 32 heads of 256
-// tokens 34.7 -> 30.4 us, 16 x 1024 63 -> 47.5).
 template <typename T, bool FP8, int D, int RW, bool HIDES>
-__global__ void __launch_bounds__(kAttnThreads, RW == 1 && D == 128 ? 4 : 1) attn_decode_kernel(AttnArgs a) {
+__global__ void __launch_bounds__(kAttnThreads, (min_ctas<T, FP8, D, RW, HIDES>())) attn_decode_kernel(AttnArgs a) {
   constexpr int DPL = D / 8;
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -618,17 +631,21 @@ IPEX_API int64_t ipex_attn_decode_counter_ints(int B, int Hkv, int G, int Sq) {
 }
 
 // CTAs of a launch with `rows` query rows per kv head (group x positions) that one SM holds at a time; 0 where the head size
-// or type is not taken.
-IPEX_API int ipex_attn_decode_ctas_per_sm(int D, int rows, int fp8_kv, int dtype) {
+// or type is not taken.  hides: some query may not see some cached key.
+IPEX_API int ipex_attn_decode_ctas_per_sm(int D, int rows, int fp8_kv, int dtype, int hides) {
   auto ask = [&](auto* tag, auto fp8, auto d) {
     using T = std::remove_pointer_t<decltype(tag)>;
     constexpr bool kF = decltype(fp8)::value;
     constexpr int kD = decltype(d)::value;
     const int r = min(kMaxRows, rows);
     const int rw = r <= 1 ? 1 : (r <= 8 && !(r > 4 && wide_rows())) ? 2 : 4;
-    const void* k = rw == 1   ? (const void*)attn_decode_kernel<T, kF, kD, 1, false>
-                    : rw == 2 ? (const void*)attn_decode_kernel<T, kF, kD, 2, false>
-                              : (const void*)attn_decode_kernel<T, kF, kD, 4, false>;
+    auto pick = [&](auto h) {
+      constexpr bool kH = decltype(h)::value;
+      return rw == 1   ? (const void*)attn_decode_kernel<T, kF, kD, 1, kH>
+             : rw == 2 ? (const void*)attn_decode_kernel<T, kF, kD, 2, kH>
+                       : (const void*)attn_decode_kernel<T, kF, kD, 4, kH>;
+    };
+    const void* k = hides ? pick(std::true_type()) : pick(std::false_type());
     int n = 0;
     const size_t sm = (size_t)(2 * kD + kAttnWarps * rw * (kD + 2) + 33 * kMaxRows) * sizeof(float);
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kAttnThreads, sm) == cudaSuccess ? n : 0;

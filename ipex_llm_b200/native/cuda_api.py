@@ -56,7 +56,7 @@ _I64_RET = {
 
 # optional entry points: declared when the library exports them (kernels added over time)
 _OPTIONAL = {
-    "ipex_attn_decode_ctas_per_sm": [ci, ci, ci, ci],
+    "ipex_attn_decode_ctas_per_sm": [ci, ci, ci, ci, ci],
     "ipex_gemm_tcgen05": [vp, vp, vp, vp, vp, ci, ci, ci, i64, i64, i64, i64, ci, vp, vp],
     "ipex_gemm_tcgen05_token_tile": [ci],
     "ipex_gemm_lowbit_tcgen05": [vp, vp, vp, vp, vp, vp, ci, ci, ci, i64, i64, i64, ci, ci, ci, vp, vp],

@@ -497,11 +497,12 @@ def _sm_count() -> int:
 
 
 @functools.lru_cache(maxsize=None)
-def _attn_ctas_per_sm(head_dim: int, rows: int, fp8: bool, dtype_code: int) -> int:
-    return max(1, int(cuda_lib().ipex_attn_decode_ctas_per_sm(head_dim, min(rows, 16), int(fp8), dtype_code)))
+def _attn_ctas_per_sm(head_dim: int, rows: int, fp8: bool, dtype_code: int, hides: bool = False) -> int:
+    return max(1, int(cuda_lib().ipex_attn_decode_ctas_per_sm(head_dim, min(rows, 16), int(fp8), dtype_code, int(hides))))
 
 
-def attn_splits(B: int, Hkv: int, kv_len: int, rows: int, head_dim: int, fp8: bool, dtype: torch.dtype) -> int:
+def attn_splits(B: int, Hkv: int, kv_len: int, rows: int, head_dim: int, fp8: bool, dtype: torch.dtype,
+                hides: bool = False) -> int:
     """KV splits of a decode attention over ``B`` sequences of ``Hkv`` kv heads with ``rows`` q rows each (GQA group x query
     length).  As many as the GPU holds CTAs of at once (a second wave doubles the launch: 8 sequences x 32 heads of 517
     tokens 17 us at 2 splits, 24 at 4), and no walk shorter than it takes to pay for handing its sums over: 160 tokens, or
@@ -511,12 +512,12 @@ def attn_splits(B: int, Hkv: int, kv_len: int, rows: int, head_dim: int, fp8: bo
     and 9.6; 8 kv heads of 8 rows, whose warps divide the rows and walk all tokens, 64 tokens 16.2, 18.9 and 17.1, 128 tokens
     21.0, 21.3 and 18.4.  Rows of 256 by fours pay from 96 tokens on: their steps are slow (a kv head of 32 such rows, 1500
     fp16 tokens 247 us in eight parts, 201 in twelve).  ``pick_nsplit``'s rule, which knows the walk's length only, where its
-    switches ask for it."""
+    switches ask for it.  ``hides``: some query may not see some cached key (a kernel of its own)."""
     if "IPEX_LLM_ATTN_STEPS" in os.environ or "IPEX_LLM_ATTN_MIN_CTAS" in os.environ:
         return pick_nsplit(B, Hkv, kv_len, rows=rows)
     heads = B * Hkv * -(-max(1, rows) // 16)
     sms = _sm_count()
-    wave = sms * _attn_ctas_per_sm(head_dim, max(1, rows), bool(fp8), api.dtype_code(dtype)) // heads
+    wave = sms * _attn_ctas_per_sm(head_dim, max(1, rows), bool(fp8), api.dtype_code(dtype), hides) // heads
     if heads >= sms:
         n = kv_len // 512
     else:
@@ -578,7 +579,7 @@ def sdpa_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask, scale: 
         q = q.contiguous()
     out = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device)
     G = Hq // Hkv
-    nsplit = attn_splits(B, Hkv, Skv, G * Sq, D, fp8, q.dtype)
+    nsplit = attn_splits(B, Hkv, Skv, G * Sq, D, fp8, q.dtype, bool(sliding_window) or (causal and Sq > 1))
     floats = lib.ipex_attn_decode_scratch_floats(B, Hkv, G, Sq, D, nsplit)
     ints = lib.ipex_attn_decode_counter_ints(B, Hkv, G, Sq)
     scratch, counters = attn_workspace(q.device, floats, ints)

@@ -124,3 +124,22 @@ def test_queries_of_any_alignment(heads, D):
     apart = torch.empty(*q.shape[:3], D + 3, dtype=q.dtype, device="cuda")[..., :D].copy_(q)
     for other in (moved, apart):
         assert torch.equal(cuda_ops.sdpa_decode(other, k, v, None, D ** -0.5, None, None), want)
+
+
+@pytest.mark.parametrize("D,rows,fp8,dtype,ctas", [
+    (64, 1, False, torch.float16, 5), (64, 1, True, torch.float16, 7), (64, 4, False, torch.float16, 4), (64, 4, True, torch.float16, 4),
+    (64, 16, False, torch.float16, 3), (64, 1, False, torch.bfloat16, 4), (64, 4, False, torch.bfloat16, 4),
+    (128, 1, False, torch.float16, 4), (128, 1, True, torch.bfloat16, 4), (128, 4, False, torch.float16, 2)])
+def test_ctas_that_an_sm_holds(D, rows, fp8, dtype, ctas):
+    """The walk waits for memory: short heads, whose registers allow it, keep their CTAs beside one another."""
+    from ipex_llm_b200.native import cuda_api as api
+    from ipex_llm_b200.ops import cuda_ops
+    assert cuda_ops._attn_ctas_per_sm(D, rows, fp8, api.dtype_code(dtype)) >= ctas
+
+
+def test_walks_that_would_spill_have_a_cta_less():
+    """One row of 128 a warp needs 168 registers in bf16, and in fp16 where keys are hidden: three CTAs, not four that spill."""
+    from ipex_llm_b200.native import cuda_api as api
+    from ipex_llm_b200.ops import cuda_ops
+    fp16, bf16 = api.dtype_code(torch.float16), api.dtype_code(torch.bfloat16)
+    assert [cuda_ops._attn_ctas_per_sm(128, 1, False, dt, h) for dt in (bf16, fp16) for h in (False, True)] == [3, 3, 4, 3]
