@@ -143,3 +143,59 @@ def test_walks_that_would_spill_have_a_cta_less():
     from ipex_llm_b200.ops import cuda_ops
     fp16, bf16 = api.dtype_code(torch.float16), api.dtype_code(torch.bfloat16)
     assert [cuda_ops._attn_ctas_per_sm(128, 1, False, dt, h) for dt in (bf16, fp16) for h in (False, True)] == [3, 3, 4, 3]
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("heads", [(4, 4, 1), (8, 2, 1), (8, 1, 3)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_rotated_queries_of_any_alignment(dtype, heads, D):
+    """New tokens behind a cache: queries, keys and rotary values that are read in runs and one by one."""
+    import ctypes
+    from ipex_llm_b200.native import cuda_api as api
+    from ipex_llm_b200.native.lib import cuda_lib, current_stream, ptr
+    from ipex_llm_b200.ops import cuda_ops
+    Hq, Hkv, Sq = heads
+    B, past, u = 2, 77, 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    g = torch.Generator(device="cuda").manual_seed(D + Hq)
+    q, kn, vn = (torch.randn(B, Sq, h, D, device="cuda", generator=g).to(dtype) for h in (Hq, Hkv, Hkv))
+    k, v = (torch.randn(B, Hkv, past + Sq, D, device="cuda", generator=g).to(dtype) for _ in range(2))
+    angle = torch.arange(past + Sq, device="cuda")[:, None] / 100.0 ** (torch.arange(D // 2, device="cuda") * 2 / D)[None]
+    cos, sin = angle.cos().contiguous(), angle.sin().contiguous()
+    lengths = torch.full((B,), past, dtype=torch.int32, device="cuda")
+    lib = cuda_lib()
+
+    def moved(t):
+        return torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t)
+
+    def run(qq, cc, ss, n):
+        kc, vc, out = k.clone(), v.clone(), torch.empty_like(q)
+        scratch, counters = cuda_ops.attn_workspace(q.device, lib.ipex_attn_decode_scratch_floats(B, Hkv, Hq // Hkv, Sq, D, n),
+                                                    lib.ipex_attn_decode_counter_ints(B, Hkv, Hq // Hkv, Sq))
+        strides = (ctypes.c_int64 * 12)(*qq.stride()[:3], *kn.stride()[:3], *kc.stride()[:3], *out.stride()[:3])
+        rc = lib.ipex_attn_decode(ptr(qq), ptr(kn), ptr(vn), ptr(kc), ptr(vc), ptr(out), ptr(lengths), 0, ptr(cc), ptr(ss),
+                                  ptr(scratch), ptr(counters), strides, B, Sq, Hq, Hkv, D, n, 1, D, 1, 0, D ** -0.5, 0.0, 0,
+                                  api.dtype_code(dtype), 0, current_stream())
+        api.check(rc, "attn_decode")
+        torch.cuda.synchronize()
+        return out, kc
+
+    def rotate(t):                                         # [B, Sq, heads, D] at positions past ..
+        c, s = cos[past:past + Sq, None].double(), sin[past:past + Sq, None].double()
+        a, b = t.double()[..., :D // 2], t.double()[..., D // 2:]
+        return torch.cat([a * c - b * s, b * c + a * s], -1)
+
+    for n in (1, 3):
+        want, kc = run(q, cos, sin, n)
+        qd = rotate(q).transpose(1, 2)
+        kd, vd = (t.double().repeat_interleave(Hq // Hkv, 1) for t in (kc, torch.cat([v[:, :, :past], vn.transpose(1, 2)], 2)))
+        hidden = torch.arange(past + Sq, device="cuda")[None] > torch.arange(past, past + Sq, device="cuda")[:, None]
+        p = torch.softmax((qd @ kd.transpose(-1, -2) * D ** -0.5).masked_fill(hidden, float("-inf")), -1)
+        # rotated queries are rounded to their type (the key that the kernel wrote is read back): every score moves by up to u
+        # times its products' magnitude, every weight by twice the largest of that
+        move = u * (qd.abs() @ kd.abs().transpose(-1, -2)).amax(-1, keepdim=True) * D ** -0.5
+        bound = (p @ vd.abs()) * (torch.expm1(2 * move) + 2.0 ** -16) + (p @ vd).abs() * u + 1e-6
+        for qq, cc, ss in ((q, cos, sin), (moved(q), cos, sin), (q, moved(cos), sin), (q, cos, moved(sin)), (moved(q), moved(cos), moved(sin))):
+            out, key = run(qq, cc, ss, n)
+            assert torch.equal(key, kc)
+            assert bool(((out.double().transpose(1, 2) - p @ vd).abs() <= bound).all())
+            assert bool(((out.double() - want.double()).abs().transpose(1, 2) <= bound).all())
