@@ -110,7 +110,7 @@ def gemv_lowbit(x: torch.Tensor, w_data: torch.Tensor, qtype: int, N: int, K: in
     if norm_weight is None and wf not in (api.WF_F16, api.WF_BF16) and _GEMV_IMPL == "stream" and act in (0, 1, 2) and \
             (act == 0 or (N % 32 == 0 and residual is None)) and K % (128 if wf in (api.WF_FP8_E4M3, api.WF_FP8_E5M2) else 64) == 0:
         from . import tcgen05_gemm
-        if tcgen05_gemm.few_faster(wf, x.dtype, M) and \
+        if tcgen05_gemm.few_faster(wf, x.dtype, M, N, K) and \
                 tcgen05_gemm.gemm_few(x, w_data, N, K, out, wf, lut=lut, bias=bias, residual=residual, act=act,
                                       pdl=pdl and _USE_PDL):
             return out
@@ -181,7 +181,7 @@ def _linear_rows(x: torch.Tensor, weight: FP4Params, M: int, N: int, K: int, wf:
     from . import tcgen05_gemm
     if not x.is_contiguous() or x.shape[1] != K:
         return None
-    few = M > GEMV_MAX_M or tcgen05_gemm.few_faster(wf, x.dtype, M)
+    few = M > GEMV_MAX_M or tcgen05_gemm.few_faster(wf, x.dtype, M, N, K)
     if M > GEMV_MAX_M and (N % 16 != 0 or os.environ.get("IPEX_LLM_TCGEN05", "1") == "0"):
         return None
     lut = lut_for(weight.qtype, x.device) if wf == api.WF_LUT4 else None

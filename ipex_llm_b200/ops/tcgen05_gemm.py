@@ -110,16 +110,37 @@ def few_exact(wf: int, dtype, rows: int) -> bool:
     return rows <= 32
 
 
-def few_faster(wf: int, dtype, rows: int) -> bool:
+def _second_round(N: int, K: int) -> bool:
+    """Whether the product for few rows begins a second round of CTAs with a handful of them (40 tiles by 8, 80 by 4 on 296
+    places), and its walks are not long enough to make up for it."""
+    tiles, split = -(-N // 128), 1
+    while split < 8 and 2 * split * tiles <= 355:       # pick_split of gemm_few.cuh
+        split *= 2
+    return split >= 4 and split * tiles > 296 and K < 8192
+
+
+def few_faster(wf: int, dtype, rows: int, N: int = 0, K: int = 0) -> bool:
     """Whether ``gemm_few`` takes one to eight rows instead of the GEMVs: it loses no precision (see ``few_exact``; minima are
-    kept apart up to 32 rows) and is faster.  The streaming GEMV of int4 and e4m3 keeps up to three rows.  us, GEMV / this, 4096
-    x 4096 | 12288 x 4096 | 4096 x 11008: int4 one row 5.5 / 5.3 | 10.2 / 11.6 | 10.1 / 10.4, four 7.3 / 5.7 | 11.7 / 11.9 | 15.4
-    / 10.6, eight 11.1 / 6.4 | 16.9 / 12.3 | -; one row in nf4 8.8 / 6.4 | 20.1 / 14.4 | 16.9 / 12.3, int8 7.4 / 6.2 | 16.1 /
-    11.9 | 14.3 / 11.2.  (Two or three rows of int4 win by themselves where N is small, and lose it again where the two kinds
-    take turns: a decode step of four layers, two sequences, 321 us with GEMVs alone and 327 with both.)"""
+    kept apart up to 32 rows) and is faster.  us, GEMV / this, 4096 x 4096 | 12288 x 4096 | 4096 x 11008 | 5120 x 5120, fp16:
+    one row: asym_int4 8.4 / 6.0 | 18.1 / 13.0 | 15.3 / 11.4 | 12.5 / 11.3, e5m2 8.3 / 6.1 | 18.3 / 11.2 | 15.6 / 10.3 | 12.0 / 11.1,
+    nf4 9.0 / 6.8 | 20.8 / 14.8 | 16.9 / 12.6 | 13.8 / 11.8, int8 7.9 / 6.5 | 17.2 / 12.0 | 14.4 / 11.3 | 11.4 / 11.4; but int8 in bf16,
+    whose codes take a conversion more, 7.9 / 7.8 | 17.3 / 16.3 | 14.4 / 14.2 | 11.5 / 12.8;
+    four rows: int4 7.8 / 6.2 | 12.1 / 12.2 | 15.9 / 10.8 | 10.6 / 11.1 (22016 x 4096 16.9 / 17.8, 28672 x 8192 34.2 / 36.6; bf16
+    17.0 / 18.5 and 34.4 / 40.4), e4m3 8.9 / 7.8 | 16.0 / 15.5 | 17.4 / 13.9 | 12.1 / 12.7 (22016 x 4096 26.1 / 23.1);
+    five rows: int4 11.7 / 6.2 | 16.5 / 12.7 | 25.2 / 10.9 | 14.9 / 11.1, e4m3 12.4 / 7.9 | 21.3 / 15.8 | 24.9 / 14.0 | 16.3 / 12.7.
+    The streaming GEMV of int4 and e4m3 keeps up to three rows.  (Two or three rows of int4 win by themselves where N is small, and
+    lose it again where the two kinds take turns: a decode step of four layers, two sequences, 321 us with GEMVs alone and 327
+    with both.  With four rows the turns pay: eight layers, four sequences, GEMVs in front of norms and this for the others 541 us,
+    GEMVs alone 572, this alone 588.)"""
     if wf == api.WF_LUT4 and dtype != torch.float16:
         return False
-    return rows >= 4 or wf not in (api.WF_SYM_INT4, api.WF_FP8_E4M3)
+    if wf == api.WF_SYM_INT4:
+        return rows > 4 or (rows == 4 and N <= 2 * K and not _second_round(N, K))
+    if wf == api.WF_FP8_E4M3:
+        return rows > 4 or (rows == 4 and not _second_round(N, K))
+    if wf == api.WF_INT8 and dtype == torch.bfloat16:
+        return rows > 3 or not _second_round(N, K)
+    return True
 
 
 def gemm_few(x: torch.Tensor, w_data: torch.Tensor, N: int, K: int, out: torch.Tensor, wf: int, lut: torch.Tensor = None,

@@ -51,3 +51,22 @@ def test_pairs_need_two_rows_for_each_token():
     o = _operands(False)
     o["w_data"] = o["w_data"][-o["w_data"].data_ptr() % 32:]
     assert tcgen05_gemm.gemm_few(o["x"], o["w_data"], N, K, o["out"], api.WF_SYM_INT4, pairs=True) is False
+
+
+def test_who_takes_one_to_eight_rows():
+    """The product for few rows where it is the faster one: measured at these sizes."""
+    from ipex_llm_b200.native import cuda_api as api
+    from ipex_llm_b200.ops.tcgen05_gemm import few_faster
+    f16, bf16 = torch.float16, torch.bfloat16
+    four = [(4096, 4096), (8192, 8192), (4096, 11008), (5120, 13824)]
+    gemv = [(22016, 4096), (28672, 8192), (5120, 5120), (10240, 4096)]
+    for dtype in (f16, bf16):
+        assert all(few_faster(api.WF_SYM_INT4, dtype, 4, *s) for s in four) and not any(few_faster(api.WF_SYM_INT4, dtype, 4, *s) for s in gemv)
+        assert few_faster(api.WF_FP8_E4M3, dtype, 4, 22016, 4096) and not few_faster(api.WF_FP8_E4M3, dtype, 4, 5120, 5120)
+        for s in four + gemv:
+            assert not any(few_faster(wf, dtype, rows, *s) for wf in (api.WF_SYM_INT4, api.WF_FP8_E4M3) for rows in (1, 2, 3))
+            assert all(few_faster(wf, dtype, 5, *s) for wf in (api.WF_SYM_INT4, api.WF_FP8_E4M3, api.WF_INT8))
+            assert few_faster(api.WF_ASYM_INT4, dtype, 1, *s) and few_faster(api.WF_FP8_E5M2, dtype, 1, *s)
+            assert few_faster(api.WF_LUT4, dtype, 1, *s) == (dtype == f16)
+    assert few_faster(api.WF_INT8, f16, 1, 5120, 5120) and few_faster(api.WF_INT8, bf16, 1, 4096, 4096)
+    assert not few_faster(api.WF_INT8, bf16, 1, 5120, 5120)
