@@ -424,3 +424,33 @@ def test_minima_of_many_stages(M, K):
             torch.cuda.synchronize()
             assert bool(((out.double() - ref).abs() <= mag * K * 2.0 ** -23 + spread + ref.abs() * U[dtype] + 1e-6).all())
     cuda_ops.check_error_flag(x.device)
+
+
+@pytest.mark.parametrize("name", ["sym_int4", "asym_int4", "nf4", "fp8_e4m3", "fp8_e5m2", "sym_int8"])
+@pytest.mark.parametrize("M,K", [(4, 8320), (5, 8320), (8, 11008)])
+def test_rows_of_every_format_between_dependent_launches(name, M, K):
+    """Where the product for few rows is the one that runs, a chain of programmatic launches whose buffers are overwritten by the
+    next round repeats one without them bit for bit."""
+    from ipex_llm_b200.ops import cuda_ops, tcgen05_gemm
+    from ipex_llm_b200.quant import qtypes
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    N, dtype = 272, torch.float16
+    assert tcgen05_gemm.few_faster(cuda_ops.QTYPE_TO_WF[qtypes.qtype_from_name(name)], dtype, M)
+    qu, pu, _ = _weights("sym_int8", K, 384, dtype, g)
+    q, packed, _ = _weights(name, N, K, dtype, g)
+    start = torch.randn(M, 384, device="cuda", generator=g).to(dtype)
+    x, y, z = (torch.empty(M, n, dtype=dtype, device="cuda") for n in (K, N, 384))
+
+    def chain(pdl):
+        z.copy_(start)
+        seen = []
+        for _ in range(6):
+            cuda_ops.gemv_lowbit(z, pu, qu, K, 384, out=x, pdl=pdl)
+            cuda_ops.gemv_lowbit(x, packed, q, N, K, out=y, residual=z[:, :N], pdl=pdl)
+            z[:, :N].copy_(y * 0.1)
+            seen.append(y.clone())
+        return torch.stack(seen)
+
+    want = chain(False)
+    assert torch.equal(chain(True), want)
+    cuda_ops.check_error_flag(x.device)
