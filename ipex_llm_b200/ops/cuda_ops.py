@@ -184,6 +184,8 @@ def _linear_rows(x: torch.Tensor, weight: FP4Params, M: int, N: int, K: int, wf:
     few = M > GEMV_MAX_M or tcgen05_gemm.few_faster(wf, x.dtype, M, N, K)
     if M > GEMV_MAX_M and (N % 16 != 0 or os.environ.get("IPEX_LLM_TCGEN05", "1") == "0"):
         return None
+    if not few and wf not in (api.WF_SYM_INT4, api.WF_FP8_E4M3):      # (the streaming GEMV's formats)
+        return None
     lut = lut_for(weight.qtype, x.device) if wf == api.WF_LUT4 else None
     out = torch.empty((M, N), dtype=x.dtype, device=x.device)
     rc = cuda_lib().ipex_linear_rows(x.data_ptr(), weight.data_ptr(), out.data_ptr(), None if lut is None else lut.data_ptr(), M, N,

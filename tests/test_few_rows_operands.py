@@ -70,3 +70,18 @@ def test_who_takes_one_to_eight_rows():
             assert few_faster(api.WF_LUT4, dtype, 1, *s) == (dtype == f16)
     assert few_faster(api.WF_INT8, f16, 1, 5120, 5120) and few_faster(api.WF_INT8, bf16, 1, 4096, 4096)
     assert not few_faster(api.WF_INT8, bf16, 1, 5120, 5120)
+
+
+def test_rows_that_only_the_general_way_takes_are_not_prepared_for(monkeypatch):
+    """bf16 code books of one to eight rows: known before an output is made or a library is asked."""
+    from ipex_llm_b200.native import cuda_api as api
+    from ipex_llm_b200.ops import cuda_ops
+
+    def asked(*a, **k):
+        raise AssertionError("prepared for a call that is refused")
+
+    for name in ("cuda_lib", "lut_for", "error_flag"):
+        monkeypatch.setattr(cuda_ops, name, asked)
+    x = torch.zeros(3, K, dtype=torch.bfloat16)
+    assert cuda_ops._linear_rows(x, None, 3, N, K, api.WF_LUT4) is None
+    assert cuda_ops._linear_rows(x, None, 3, 5120, K, api.WF_INT8) is None
