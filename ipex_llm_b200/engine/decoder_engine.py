@@ -461,11 +461,13 @@ class DecoderEngine:
             api.check(rc, "embedding")
         # (later pipeline stages: the previous stage's hidden states were received into h[0][:B])
         if B <= 24 and self._few_decode_ok() and B >= self._few_from:
-            # some sequences (formats without a streaming GEMV: any number): the weights are read once per step (eight-row GEMVs read them once per group of eight, and work
-            # the rows up in every CTA).  The normalised rows come as value and remainder and the products multiply by the codes
-            # themselves (a code book's values in fp16, as the GEMVs), so nothing is rounded that the GEMVs would not round.
+            # some sequences (formats without a streaming GEMV: any number): the weights are read once per step (eight-row GEMVs
+            # read them once per group of eight, and work the rows up in every CTA).  The normalised rows come as value and
+            # remainder and the products multiply by the codes themselves (a code book's values in fp16, as the GEMVs), so
+            # nothing is rounded that the GEMVs would not round.
             # Llama-2-7B sym_int4, 8 sequences of 517 tokens: 3.15 -> 2.74 ms per step; four of its layers, one sequence of 512
-            # tokens, nf4: 477 -> 403 us, sym_int8: 422 -> 364; four sequences, nf4: 541 -> 422, but sym_int4: 351 -> 362.
+            # tokens, nf4: 477 -> 403 us, sym_int8: 422 -> 364; four sequences, nf4: 541 -> 422, but sym_int4: 351 -> 362 (eight
+            # layers: GEMVs in front of norms and this for o and down, as ``gemv_lowbit`` has it, 541, this for all 588).
             def pairs(h, w):
                 return cuda_ops.rms_norm_pairs(h, w, self.eps, pdl=self.use_pdl)
             for L in self.layers:

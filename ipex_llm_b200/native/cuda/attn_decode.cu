@@ -116,8 +116,9 @@ struct RawKV {
 // One row of 128: four, 128 registers, where that does not spill (fp16: 32 sequences x 32 heads of 256 tokens 31.0 with 0 and 28.5,
 // of 2048 182 and 165; e5m2, 8 x 517 tokens 14.5 and 13.8).  bf16 caches and hidden fp16 keys spill under it (2048 bf16 tokens 184
 // with 0 and 294, 1024 fp16 tokens with a window 104 and 120).
-// Heads of 64 wait for memory and want the warps: 32 x 32 heads of 1024 fp16 tokens 51.9 / 59.2, e5m2 34.4 / 38.5; 8 queries to each
-// of 8 x 32 heads 79.4 / 102.
+// Heads of 64 wait for memory and want the warps: 32 x 32 heads of 1024 fp16 tokens 51.9 / 59.2, e5m2 34.4 / 38.5; 8 queries to
+// each of 8 x 32 heads 79.4 / 102.  (Not where few heads leave the SMs room: 8 heads of 4 rows, 1024 fp16 tokens 13.3 / 11.9, 8 x 4
+// heads of 16 rows 37.4 / 34.4.)
 // Everything else is the faster for its registers, though an SM holds a CTA less: 32 x 8 heads of 128 with 4 rows, 1024 e5m2
 // tokens 47.9 / 44.9, bf16 68.8 / 64.3, 8 x 32 x 4 queries fp16 80.9 / 72.1; 8 x 16 heads of 256 33.5 / 30.9, e5m2 23.2 / 21.6.
 template <typename T, bool FP8, int D, int RW, bool HIDES> constexpr int min_ctas() {

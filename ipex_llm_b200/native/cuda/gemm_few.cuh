@@ -1,12 +1,12 @@
-// Products of 1 to 64 token rows with packed weights (decode steps of a batch, drafted continuations), most of those with up to
-// 24 rows by this kernel, the others by gemm_few_tcgen05.cuh:
+// Products of 1 to 64 token rows with packed weights (decode steps of a batch, drafted continuations): those with up to 24 rows
+// (16 with minima), and more where two of them make a token, by this kernel, the others by gemm_few_tcgen05.cuh:
 //     out[M, N] = x[M, K] . W[N, K]^T  (+ bias) (+ residual)   or   act(gate) * up  for interleaved gate/up rows
 //
 // What bounds it: with so few rows the weights' codes have to be taken apart as fast as they arrive, some nine instructions
 // for eight codes, and each is used for a few columns only.  So a warp keeps everything to itself: it reads the packed codes
-// of 64 weight rows from a ring in shared memory, makes them 16-bit operands in the registers of the very lane that the
+// of 32 weight rows from a ring in shared memory, makes them 16-bit operands in the registers of the very lane that the
 // matrix instruction wants them in (the packed layout was made for that: a lane's 16 bytes are consecutive k of one row), and
-// multiplies them by token fragments that it loads once for its 64 rows.  No expanded weight is written anywhere, and no other
+// multiplies them by token fragments that it loads once for its 32 rows.  No expanded weight is written anywhere, and no other
 // warp is waited for before the sums are added up.
 //
 // The codes themselves are multiplied (small integers, fp8 values: exact in 16 bits; a code book's values are rounded to 16
@@ -15,8 +15,8 @@
 //
 // A CTA holds a tile of 128 weight rows over a share of k, two CTAs fit an SM (one loads or adds up while the other
 // multiplies), and a cluster of up to eight CTAs shares the k of a tile: the parts meet through distributed shared memory, in
-// a fixed order.  One warp fills the ring: the weights' part of the first stages is asked for before the kernel in front has
-// ended.
+// a fixed order.  The weights' part of the ring's first stages is asked for before the kernel in front has ended; later the warps
+// take turns at filling it.
 //
 // Measured (us per launch between dependent launches, weights from memory; a tcgen05 form that wrote expanded weights to shared
 // memory -> this one): int4, 16 rows, 12288 x 4096 19.4 -> 14.6, 22016 x 4096 32.5 -> 22.1, 32000 x 4096 39.7 -> 23.6.  ncu, 32000
@@ -25,7 +25,7 @@
 //
 // x may hold two rows per token (2m: the value rounded to 16 bits, 2m + 1: what that left over); their products are added in
 // 32 bits at the end.
-// Every wait is bounded (error codes 20 loader, 22 multiplying warps).
+// Every wait is bounded (error code 22).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -134,7 +134,8 @@ __device__ __forceinline__ uint4 codes4(uint32_t w, const uint32_t* book, const 
   } else if constexpr (!CODES) {
     return expand4<T, WF>(w, sc, nullptr);
   } else if constexpr (std::is_same<T, __half>::value) {
-    // 1024 + q, and 1024 + 16 q for the nibbles above: a shift for every other pair only
+    // 1024 + q, and 1024 + 16 q for the nibbles above: a shift for every other pair only (integers placed in the last bits of a
+    // number of known exponent: Kim et al., "Who Says Elephants Can't Run", 2022)
     const uint32_t u = w >> 8;
     const __half2 off = __float2half2_rn(1024.f + zero), sixteenth = __float2half2_rn(0.0625f),
                   off16 = __float2half2_rn(-64.f - zero);
@@ -296,8 +297,8 @@ template <typename T> __device__ __forceinline__ void fill_book(uint32_t* book, 
 // infinite token the codes' part and the minimum's are infinities of any signs, or a zero code's product with it, where the
 // weight's own product is an infinity of the weight's sign.  Only rows with such a token (or without a number) come here.
 template <typename T, int PARTS, int COLS>
-__device__ __noinline__ void add_up_again(const uint8_t* w, const T* x, int64_t ldx, int rows, int N, int chunks, float* red, int tile, int k0,
-                                          int k1) {
+__device__ __noinline__ void add_up_again(const uint8_t* w, const T* x, int64_t ldx, int rows, int N, int chunks, float* red,
+                                          int tile, int k0, int k1) {
   constexpr int kPitch = kBM + 4;
   const int row = threadIdx.x % kBM, n = tile * kBM + row;
   if (n >= N) return;
@@ -316,7 +317,8 @@ __device__ __noinline__ void add_up_again(const uint8_t* w, const T* x, int64_t 
                                                                ((k >> 3) & 1) * 4);
       const __half* d = reinterpret_cast<const __half*>(scales + chunk * 64) + h * 16 + pair_row(n & 15);
       const float m = __half2float(d[row_tiles * chunks * 32]);
-      again = fmaf(fmaf(__half2float(*d), (float)((word >> (4 * ((e >> 1) + 4 * (e & 1)))) & 15), m), to_float(x[c * ldx + k]), again);
+      const float code = (float)((word >> (4 * ((e >> 1) + 4 * (e & 1)))) & 15);
+      again = fmaf(fmaf(__half2float(*d), code, m), to_float(x[c * ldx + k]), again);
     }
     for (int p = 0; p < PARTS; ++p) sum[p * COLS * kPitch] = p == 0 ? again : 0.f;
   }
@@ -555,17 +557,19 @@ int launch(const Operands& o, Args a, cudaStream_t st, bool pdl, int asked) {
   return launch_tiles<T, C::kCodes, C::kPlanes, C::kCols, C::WK>(kernel<T, WF, NT, WN>, limit, C::kSmem, o, a, st, pdl);
 }
 
+// The instances that ipex_gemm_few's rule leaves to this kernel.
 template <typename T, int WF>
 int by_columns(const Operands& o, const Args& a, cudaStream_t st, bool pdl, int asked) {
-  switch ((a.rows + 7) / 8) {
-    case 1: return launch<T, WF, 1, 1>(o, a, st, pdl, asked);
-    case 2: return launch<T, WF, 2, 1>(o, a, st, pdl, asked);
-    case 3: return launch<T, WF, 3, 1>(o, a, st, pdl, asked);
-    case 4: return launch<T, WF, 4, 1>(o, a, st, pdl, asked);
-    case 5:
-    case 6: return launch<T, WF, 3, 2>(o, a, st, pdl, asked);
-    default: return launch<T, WF, 4, 2>(o, a, st, pdl, asked);
+  const int cols = (a.rows + 7) / 8;
+  if (cols == 1) return launch<T, WF, 1, 1>(o, a, st, pdl, asked);
+  if (cols == 2) return launch<T, WF, 2, 1>(o, a, st, pdl, asked);
+  if constexpr (WF != WF_ASYM_INT4)
+    if (cols == 3) return launch<T, WF, 3, 1>(o, a, st, pdl, asked);
+  if constexpr (WF != WF_FP8_E4M3 && WF != WF_FP8_E5M2) {      // pairs
+    if (cols == 5 || cols == 6) return launch<T, WF, 3, 2>(o, a, st, pdl, asked);
+    if (cols > 6) return launch<T, WF, 4, 2>(o, a, st, pdl, asked);
   }
+  return (int)cudaErrorInvalidValue;
 }
 
 template <typename T>

@@ -9,7 +9,9 @@
 // through shared memory.  us per launch between dependent launches, weights from memory, gemm_few.cuh's form | this: int4, 24
 // rows, 22016 x 4096 25.8 | 30, 32 rows 33.5 | 29.4, 64 rows 59.7 | 39.1, 32000 x 4096 at 64 rows 70.7 | 34.7; nf4, 40 rows,
 // 22016 x 4096 51.7 | 36.4; fp8 48.4 | 38.3.  (A form that wrote expanded weights to shared memory took 42.5, 55.5 and 65.9 for
-// int4 at 32 and 64 rows, 67 for nf4 at 64.)
+// int4 at 32 and 64 rows, 67 for nf4 at 64.)  Columns of 64 of the 8-bit floats spill some 50 to 150 bytes a thread beside two
+// CTAs' registers, and are the faster all the same: 64 rows, 22016 x 4096, that form and this: e4m3 fp16 64.2 and 48.5, bf16 64.2
+// and 49.1, e5m2 62.3 and 48.3, 64.1 and 49.1.
 //
 // Up to 32 columns (and in the 8-bit float formats) the codes are multiplied and the sums of each scale group scaled and added
 // in 32 bits.  More columns of the other formats are expanded and scaled in 16 bits, as in the kernel for many rows, and the sums
@@ -18,8 +20,8 @@
 // Minima up to 32 columns stay apart too: their part is their product with the sums of the tokens, which a team makes (eight
 // tokens a warp, products with ones) and adds while its products run: the sums of a stage behind its barrier, their product with
 // the minima behind the next one's.  Sums by gemm_few.cuh's way (every warp makes all of them) and this, us at 24 | 32 rows of
-// fp16: 12288 x 4096 24.8 / 22.7 | 32.3 / 23.5, 4096 x 11008 20.2 / 18.4 | 26.0 / 18.9, 22016 x 4096 36.5 / 35.4 | 47.8 / 36.9 (bf16
-// 46.9 / 38.4); weights expanded and scaled in 16 bits (in a form before these) took 22.3, 19.2 and 34.6 at 32 rows.  (The minima's
+// fp16: 12288 x 4096 24.8 / 22.7 | 32.3 / 23.5, 4096 x 11008 20.2 / 18.4 | 26.0 / 18.9, 22016 x 4096 36.5 / 35.4 | 47.8 / 36.9
+// (bf16 46.9 / 38.4); weights expanded and scaled in 16 bits (in a form before these) took 22.3, 19.2 and 34.6 at 32 rows.  (The minima's
 // product at the end, as tf32, instead of stage by stage: 24.1, 20.4 and 38.4.)
 //
 // A CTA holds 128 weight rows over a share of k; two teams of four warps take its stages of 128 k in turn, and two CTAs fit an SM,
@@ -56,7 +58,8 @@ template <int WF, int N> struct Cfg {
   static constexpr int kStagesFit = (kSmemMax - 1024 - kTail) / kStageBytes;
   static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;
   static constexpr int kSmem = 1024 + kStages * kStageBytes + kTail;
-  static_assert(kStages > kTeams && kRedBytes <= kStages * kStageBytes && groups * N <= kTeamCols - 64 && (!minima || N == 32), "ring");
+  static_assert(kStages > kTeams && kRedBytes <= kStages * kStageBytes && groups * N <= kTeamCols - 64, "ring");
+  static_assert(!minima || N == 32, "eight tokens to each of a team's warps");
 };
 
 __device__ __forceinline__ void tmem_st_32(uint32_t taddr, const uint32_t (&v)[32]) {
@@ -288,7 +291,8 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
       if (ok) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          xb[i] = *reinterpret_cast<const uint4*>(st + C::kXAt + (i >> 1) * C::kPiece + qd * 1024 + g * 128 + (((2 * t + (i & 1)) ^ g) << 4));
+          xb[i] = *reinterpret_cast<const uint4*>(st + C::kXAt + (i >> 1) * C::kPiece + qd * 1024 + g * 128 +
+                                                  (((2 * t + (i & 1)) ^ g) << 4));
       }
     }
     tcgen05_fence_before();
@@ -320,7 +324,8 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
             mma16<T>(s, one, one, one, one, xb[2 * h + o].x, xb[2 * h + o].y);
             mma16<T>(s, one, one, one, one, xb[2 * h + o].z, xb[2 * h + o].w);
           }
-          if (lane < 4) *reinterpret_cast<float2*>(sums + ((team * 2 + turn) * 2 + h) * N + 8 * qd + 2 * lane) = make_float2(s[0], s[1]);
+          float* to = sums + ((team * 2 + turn) * 2 + h) * N + 8 * qd;
+          if (lane < 4) reinterpret_cast<float2*>(to)[lane] = make_float2(s[0], s[1]);
         }
       }
       dm[0] = mn[0];
