@@ -225,7 +225,7 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
   for (int i = team; i < nst; i += kTeams) {
     if (waiting) {
       if (ok) ok = warp_wait(&done[team], dph, abort_flag);
-      dph ^= 1;
+      if (ok) dph ^= 1;
       tcgen05_fence_after();
       if (ok && issuer && i - kTeams + S < nst) {
         load_weights(i - kTeams + S, last, last_use + 1);
@@ -333,10 +333,12 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
       turn ^= 1;
     }
     waiting = true;
-    last = slot;
-    last_use = use;
-    slot += kTeams;
-    if (slot >= S) { slot -= S; ++use; }
+    if (ok) {                                       // (a wait that ran out: the barriers behind the loop are those of its stage)
+      last = slot;
+      last_use = use;
+      slot += kTeams;
+      if (slot >= S) { slot -= S; ++use; }
+    }
   }
   if (waiting) {
     if constexpr (C::minima) {
@@ -358,7 +360,10 @@ kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtenso
   if (!ok) {
     if (lane == 0) report(a.err, 24);
     mbar_wait_quiet(&done[team], dph, 1 << 12);     // products and copies in flight
-    for (int s = 0; s < 2 * S; ++s) mbar_wait_quiet(&full[s], (use >> 1) & 1, 1 << 10);
+    for (int s = 0; s < S; ++s) {
+      const int u = s < slot ? use + 1 : use;
+      mbar_wait_quiet(barrier(s, u), (u >> 1) & 1, 1 << 10);
+    }
   }
   tcgen05_fence_before();
   __syncthreads();                                  // the ring has been read, and every copy has landed
