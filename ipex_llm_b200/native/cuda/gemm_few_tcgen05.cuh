@@ -20,8 +20,8 @@
 // Minima up to 32 columns stay apart too: their part is their product with the sums of the tokens, which a team makes (eight
 // tokens a warp, products with ones) and adds while its products run: the sums of a stage behind its barrier, their product with
 // the minima behind the next one's.  Sums by gemm_few.cuh's way (every warp makes all of them) and this, us at 24 | 32 rows of
-// fp16: 12288 x 4096 24.8 / 22.7 | 32.3 / 23.5, 4096 x 11008 20.2 / 18.4 | 26.0 / 18.9, 22016 x 4096 36.5 / 35.4 | 47.8 / 36.9
-// (bf16 46.9 / 38.4); weights expanded and scaled in 16 bits (in a form before these) took 22.3, 19.2 and 34.6 at 32 rows.  (The minima's
+// fp16: 12288 x 4096 24.8 / 22.3 | 32.3 / 23.1, 4096 x 11008 20.2 / 18.4 | 26.0 / 18.9, 22016 x 4096 36.5 / 35.1 | 47.8 / 36.6
+// (bf16 46.9 / 37.5); weights expanded and scaled in 16 bits (in a form before these) took 22.3, 19.2 and 34.6 at 32 rows.  (The minima's
 // product at the end, as tf32, instead of stage by stage: 24.1, 20.4 and 38.4.)
 //
 // A CTA holds 128 weight rows over a share of k; two teams of four warps take its stages of 128 k in turn, and two CTAs fit an SM,

@@ -4,7 +4,7 @@ Counterparts of the reference's ``LowBitLinear``, ``MatMulLowBit``, ``MatMulLowB
 ``BF16Linear`` and their vLLM variants (python/llm/src/ipex_llm/transformers/low_bit_linear.py:500-908).
 
 Dispatch on a CUDA tensor (always the package's own sm_100a kernels, never a silent eager fallback):
-  M <= 64 rows  -> streaming GEMV (up to three rows of int4 and e4m3) or the product for few rows, in one native call
+  M <= 64 rows  -> streaming GEMV (up to three or four rows of int4 and e4m3) or the product for few rows, in one native call
   M  > 64 rows  -> tcgen05/TMEM GEMM with in-kernel dequantization
 On the CPU the packed canonical blocks go through the host library's low-bit matmul.
 """
